@@ -1,6 +1,7 @@
 // bptt.hpp -- the differentiable mode (see bptt.cu for the model).
 #pragma once
 
+#include <cuda_runtime.h>
 #include <stddef.h>
 
 #include <vector>
@@ -10,36 +11,48 @@ namespace nemo_b200 {
 // sizes and synapse structure (shared by both state types)
 struct BpttDev {
 	int N, B, T, R, ckpt, smooth;
-	const int* inStart;   // [N+1] in-synapses by target
-	const int* inSrc;
-	const int* inDelay;
-	const int* inSyn;     // synapse index (into W)
-	const int* outStart;  // [N+1] out-synapses by source (synapse index = position)
-	const int* outTgt;
-	const int* outDelay;
+	int groups;           // trial groups of BPTT_GROUP trials (the last one may be smaller)
+	int lanes;            // trials of a group rounded up to a power of two
+	int wordLog;          // log2 of a spike word's bytes: 4 bits per trial of a group
+	// in-synapses by target, in synapse order, as {source, delay}, delays
+	// clamped to T (a longer one never arrives); [N+1] and the synapse index
+	const int* inStart;
+	const int2* inSd;
+	const int* inSyn;
+	int ring;             // the longest delay: ms of spikes that a gather reads
+	int maskStride;       // bytes of a slice of spike masks: a header, then a mask of `lanes` bits per neuron
+	// out-synapses by source, each source's synapses of delay >= 2 before
+	// those of delay 1 (outMid), as offsets of their target's trials `delay`
+	// ms later in lamI: delay x N x B + target x B
+	const int* outStart;  // [N+1] also the synapse range of a source: its weights are W[outStart[n] ..]
+	const int* outMid;
+	const int* outPad;    // [N+1] start of a source's lists in shared memory, each list padded to four entries
+	const unsigned long long* outOff;
+	const int* outSyn;    // synapse index
 };
 
 // state, trajectory and adjoint arrays in the state type Real
 template<typename Real>
 struct BpttState {
 	Real alpha, lossScale;
-	Real* S;              // [N][T][B]
-	Real* v;              // [N][B]
-	Real* u;
+	unsigned char* words; // [T][groups][N] spike counts of a group's trials, 4 bits each (hard threshold)
+	unsigned char* masks; // [T][groups] slices of maskStride bytes: header (some neuron fired more than once), fired bits
+	Real* S;              // [T][N][B] spikes (smooth threshold only)
+	Real* I;              // [T][N][B] synaptic input + noise of the last forward pass
 	Real* ckV;            // [nck][N][B]
 	Real* ckU;
-	Real* r;              // [R][B]
-	Real* rHist;          // [R][T][B]
-	Real* lossPart;       // [N][B]
-	Real* segV;           // [ckpt][N][B]
+	Real* rHist;          // [T][R][B]
+	Real* lossPart;       // [R][B]
+	Real* segV;           // [ckpt][N][B] start states of the segment being differentiated
 	Real* segU;
-	Real* segSyn;
-	Real* lamV;           // [N][B]
-	Real* lamU;
-	Real* lamR;           // [R][B]
-	Real* lamI;           // [N][T][B]
+	Real* lamI;           // [T][N][B]
+	Real* lamU;           // [N][B] adjoint of the initial u
 	Real* gA;             // [N][B]
 	Real* gB;
+	Real* scratch;        // per-item arrays of the two loops when they do not fit in shared memory
+	float* listW;         // [M] weights in list order, likewise
+	unsigned* sync;       // barrier counters of the loops and the flag words (bptt.cu)
+	unsigned* hostError;  // mapped host word: a barrier wait gave up
 };
 
 // the caller's float32 tensors (device pointers)
@@ -71,19 +84,39 @@ public:
 	unsigned neurons() const { return (unsigned) D.N; }
 
 private:
+	// launch shape of the forward or the backward loop: CTAs per trial
+	// group, neurons per CTA, groups per launch, shared memory, and what
+	// lives there (0: nothing; 1: the CTA's synapses and per-item arrays; 2:
+	// and the forward loop's window of spike masks)
+	struct Loop {
+		int ctas = 1, cells = 1, groups = 1, mode = 0;
+		size_t smem = 0;
+	};
 	BpttDev D;
 	bool m_fp64 = false;
 	BpttState<float> X32{};
 	BpttState<double> X64{};
+	Loop m_fwd, m_bwd;
+	int m_maxGroups = 1;   // trial groups of one launch at most
+	size_t m_limit = 0;    // dynamic shared memory of a loop's CTA at most
+	unsigned* m_hostError = nullptr;  // mapped pinned
 	int m_device = 0;
 	size_t m_M = 0;
 	std::vector<void*> m_allocs;
+	void release() noexcept;
 	void* alloc(size_t bytes);
-	const int* upload(const std::vector<int>& v);
+	template<typename V> const V* upload(const std::vector<V>& v);
+	Loop planLoop(const std::vector<int>& start, int itemArrays, int minCells, size_t realSize, int sms,
+			const size_t entry[3], size_t window) const;
+	void checkError();
 	template<typename Real> void allocState(BpttState<Real>& X);
 	template<typename Real> void forwardT(BpttState<Real>& X, const BpttParams& P, float* loss, void* stream);
 	template<typename Real> void backwardT(BpttState<Real>& X, const BpttParams& P, float* dW, float* da,
 			float* db, void* stream);
+	template<typename Real> void launchLoop(const Loop& p, const void* kernel, BpttState<Real>& X, const BpttParams& P,
+			cudaStream_t st);
+	template<typename Real> const void* forwardKernel() const;
+	template<typename Real> const void* backwardKernel() const;
 	template<typename Real> void readoutT(BpttState<Real>& X, float* out, void* stream);
 };
 

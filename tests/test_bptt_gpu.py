@@ -201,3 +201,80 @@ def test_full_size_accuracy_vs_fp64_autograd():
     assert lerr32 <= TOL
     for e, t in zip(e32, torch32):
         assert e <= max(TOL, 2.0 * t), (e32, torch32)
+
+
+# (neurons, fanout, ms, trials, readout, noise scale): a lane's 1 to 4 trials,
+# groups of 16 (17, 33 trials), one neuron, fewer neurons than warps, more
+# than a CTA's warps hold, lists and windows beyond shared memory, and noise
+# so strong that neurons fire several times in a ms
+LOOP_SHAPES = [(1, 1, 12, 1, 1, 1.0), (7, 3, 30, 2, 7, 1.0), (33, 9, 30, 3, 5, 1.0), (130, 17, 40, 5, 10, 1.0),
+               (100, 40, 30, 8, 10, 1.0), (64, 64, 25, 13, 64, 1.0), (90, 20, 25, 17, 9, 1.0), (65, 33, 20, 33, 8, 1.0),
+               (2100, 5, 15, 6, 40, 1.0), (40, 2500, 12, 4, 8, 1.0), (40, 30000, 12, 2, 8, 0.2), (60, 20, 20, 16, 10, 60.0),
+               (60, 20, 20, 3, 10, 60.0)]
+
+
+@pytest.mark.parametrize("state_dtype", [torch.float64, torch.float32])
+@pytest.mark.parametrize("shape", LOOP_SHAPES)
+def test_loops_match_autograd_at_their_edges(shape, state_dtype):
+    """Loss and gradients of the hard threshold over the shapes of the
+    forward and adjoint loops, with targets away from the trains (a loss that
+    vanishes has no relative error).  float64 state: TOL.  float32 state: no
+    worse than twice PyTorch's own float32 autograd, as above."""
+    neurons, fanout, ms, trials, readout, scale = shape
+    dev, net, model, noise, target = setup(neurons=neurons, fanout=fanout, ms=ms, trials=trials, readout=readout,
+                                           smooth=False, ckpt=7, state_dtype=state_dtype)
+    noise, target = noise * scale, target + 1.0
+    W, a, b = net.tensors(dev)
+    loss = model.loss(W, a, b, noise, target)
+    loss.backward()
+    l64, gW, ga, gb = reference(net, dev, noise, target, readout, False)
+    ours = [relerr(loss.detach(), l64), relerr(W.grad, gW), relerr(a.grad, ga), relerr(b.grad, gb)]
+    bound = [TOL] * 4
+    if state_dtype == torch.float32:
+        l32, tW, ta, tb = reference(net, dev, noise, target, readout, False, dtype=torch.float32)
+        bound = [max(TOL, 2.0 * e) for e in (relerr(l32, l64), relerr(tW, gW), relerr(ta, ga), relerr(tb, gb))]
+    assert all(e <= t for e, t in zip(ours, bound)), (ours, bound)
+
+
+def test_a_weight_that_is_not_finite_reaches_its_target_without_a_spike():
+    """inf x 0 is NaN: the target's state is NaN from the first delivery on
+    (so it never fires and the loss stays finite), and so is the gradient of
+    every weight into it, whether or not the source fired."""
+    dev, net, model, noise, target = setup(neurons=40, fanout=8, ms=20, trials=4, readout=40, smooth=False,
+                                           state_dtype=torch.float64)
+    W, a, b = net.tensors(dev)
+    with torch.no_grad():
+        W[5] = float("inf")
+    loss = model.loss(W, a, b, 0 * noise, target)  # no noise: nothing fires
+    loss.backward()
+    into = torch.as_tensor(net.target == net.target[5], device=dev)
+    assert bool(torch.isfinite(loss)) and bool(torch.isnan(W.grad[into]).all())
+    with torch.no_grad():
+        W[5] = 0.1
+    W.grad = None
+    model.loss(W, a, b, noise, target).backward()  # the next pass is not affected
+    assert bool(torch.isfinite(W.grad).all())
+
+
+def test_loops_under_graph_capture():
+    """Forward and backward captured in a CUDA graph and replayed on other
+    inputs give the eager results."""
+    dev, net, model, noise, target = setup(neurons=300, fanout=20, ms=30, trials=4, readout=20, smooth=False,
+                                           state_dtype=torch.float64)
+    W, a, b = net.tensors(dev, requires_grad=False)
+    other = noise.flip(1).contiguous()
+    want = (model.forward_raw(W, a, b, other, target),) + model.backward_raw(W, a, b, other, target)
+    want = [x.clone() for x in want]
+    stream = torch.cuda.Stream()
+    stream.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(stream):
+        model.forward_raw(W, a, b, noise, target)
+    torch.cuda.current_stream().wait_stream(stream)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = (model.forward_raw(W, a, b, noise, target),) + model.backward_raw(W, a, b, noise, target)
+    for _ in range(2):
+        noise.copy_(other)
+        graph.replay()
+        torch.cuda.synchronize()
+        assert all(torch.equal(x, y) for x, y in zip(got, want))
