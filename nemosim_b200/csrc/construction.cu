@@ -216,6 +216,13 @@ T* upload(Scratch& scratch, const T* host, size_t n, cudaStream_t st)
 	return d;
 }
 
+__global__ void rank_kernel(size_t S, const uint32_t* src, const uint32_t* rank, uint32_t* key)
+{
+	for(size_t k = (size_t) blockIdx.x * blockDim.x + threadIdx.x; k < S; k += (size_t) gridDim.x * blockDim.x) {
+		key[k] = rank[src[k]];
+	}
+}
+
 } // namespace
 
 void construct_on_device(DeviceConstruction& c, cudaStream_t st)
@@ -360,6 +367,40 @@ void construct_on_device(DeviceConstruction& c, cudaStream_t st)
 	}
 	CC_CUDA(cudaStreamSynchronize(st));
 	c.dlvGroups = hg;
+}
+
+uint32_t* weight_order(size_t S, const uint32_t* src, const uint32_t* pos, const std::vector<uint32_t>& rank,
+		cudaStream_t st)
+{
+	// everything at once, so that a lack of memory leaves nothing behind
+	void* p[5] = {};
+	int bits = 1;
+	while(bits < 32 && (1ull << bits) < rank.size()) ++bits;
+	size_t tmpBytes = 0;
+	uint32_t* none = nullptr;
+	CC_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tmpBytes, none, none, none, none, (int) S, 0, bits, st));
+	const size_t bytes[5] = { S * 4, S * 4, S * 4, rank.size() * 4, std::max<size_t>(tmpBytes, 1) };
+	bool ok = true;
+	for(int i = 0; i < 5 && ok; ++i) ok = cudaMalloc(&p[i], bytes[i]) == cudaSuccess;
+	if(!ok) {
+		cudaGetLastError();
+		for(void* q : p) cudaFree(q);
+		return nullptr;
+	}
+	auto* order = static_cast<uint32_t*>(p[0]);
+	auto* key = static_cast<uint32_t*>(p[1]);
+	auto* sorted = static_cast<uint32_t*>(p[2]);
+	auto* ranks = static_cast<uint32_t*>(p[3]);
+	cudaError_t err = cudaMemcpyAsync(ranks, rank.data(), bytes[3], cudaMemcpyHostToDevice, st);
+	if(err == cudaSuccess) {
+		rank_kernel<<<blocks(S), THREADS, 0, st>>>(S, src, ranks, key);
+		err = cub::DeviceRadixSort::SortPairs(p[4], tmpBytes, key, sorted, pos, order, (int) S, 0, bits, st);
+	}
+	if(err == cudaSuccess) err = cudaStreamSynchronize(st);
+	for(int i = 1; i < 5; ++i) cudaFree(p[i]);
+	if(err != cudaSuccess) cudaFree(order);
+	CC_CUDA(err);
+	return order;
 }
 
 uint64_t device_digest(const void* p, size_t bytes, cudaStream_t st)

@@ -74,6 +74,12 @@ struct DeviceConstruction {
 // host build does, for the first such synapse in insertion order.
 void construct_on_device(DeviceConstruction& c, cudaStream_t stream);
 
+// The forward positions of S synapses (src: local source, pos: position, in
+// insertion order, on the device) by ascending rank[source] (a host array),
+// insertion order within a source: cudaMalloc'd, null when memory is short.
+uint32_t* weight_order(size_t S, const uint32_t* src, const uint32_t* pos, const std::vector<uint32_t>& rank,
+		cudaStream_t stream);
+
 // A digest of a device array (position-dependent hash of its bytes, summed)
 uint64_t device_digest(const void* p, size_t bytes, cudaStream_t stream);
 

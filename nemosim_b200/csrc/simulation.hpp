@@ -338,8 +338,26 @@ private:
 	cudaGraphExec_t m_graph = nullptr;
 	uint32_t m_graphP = 0, m_graphT = 0;
 	unsigned long long* m_hCycle = nullptr;
-	size_t decodeBatchStep(uint32_t r, unsigned step, unsigned* counts, unsigned* ids, size_t pos, size_t cap);
-	std::vector<std::vector<uint32_t>> m_batchScratch;
+	// the results of run() (collect_kernel): per-step counters and ids in
+	// mapped host memory, and for a batch its stream order (null: local
+	// order) and the network at each position of it
+	void collect(uint64_t first, unsigned chunk, unsigned begin, bool ids, bool perNet);
+	uint32_t* m_hStage = nullptr;    // mapped pinned: results on their way to the caller
+	uint32_t* m_dStage = nullptr;
+	size_t m_stageCap = 0;           // words
+	uint64_t* m_hSteps = nullptr;    // mapped pinned: events [R], STDP entries [R], fired counts [R] u32, error word
+	uint64_t* m_dSteps = nullptr;
+	const uint64_t* stepEventCounts() const { return m_hSteps; }
+	const uint32_t* stepCounts() const { return reinterpret_cast<const uint32_t*>(m_hSteps + 2 * (size_t) m_dev.R); }
+	const uint32_t* stepError() const { return stepCounts() + m_dev.R; }
+	uint32_t* m_streamOrder = nullptr;
+	uint32_t* m_streamNet = nullptr;
+	uint32_t* m_netCounts = nullptr; // [R][nets]
+	// weights in network iteration order
+	uint32_t* m_weightOrder = nullptr;
+	bool ensureWeightOrder();
+	void hostWeights(int32_t* out);
+	std::vector<unsigned> sourcesByGlobalId() const;
 	unsigned m_deliverGrid = 1184;  // CTAs of deliver_kernel
 	unsigned m_applyGrid = 1184;    // CTAs of apply_kernel
 	uint32_t m_P = 256, m_T = 256;
@@ -383,7 +401,7 @@ private:
 	std::chrono::steady_clock::time_point m_timerStart;
 
 	// host staging
-	uint32_t* m_hFired = nullptr;  // pinned, [R][W]
+	uint32_t* m_hFired = nullptr;  // pinned [W]: stepNoAlloc's fired words
 	uint32_t* m_hStim = nullptr;   // mapped pinned stimulus staging of step()
 	uint32_t* m_dStimMapped = nullptr;
 	size_t m_stimCap = 0;
