@@ -8,12 +8,14 @@
 
 namespace nemo_b200 {
 
-// wfx_toFloat with saturation (src/nemo/fixedpoint.cpp:40-49)
+// wfx_toFloat with saturation (src/nemo/fixedpoint.cpp:40-49): the clamped sum
+// over 2^20.  The clamped value fits an int, and scaling by a power of two is
+// exact (its magnitude is 0 or at least 2^-20), so a 32-bit conversion and a
+// multiplication give the bits of the division.
 __device__ __forceinline__ float wfx_to_float(long long v)
 {
-	v = v > (long long) INT32_MAX ? (long long) INT32_MAX : v;
-	v = v < (long long) INT32_MIN ? (long long) INT32_MIN : v;
-	return __fdiv_rn(__ll2float_rn(v), 1048576.0f);
+	const int c = v > (long long) INT32_MAX ? INT32_MAX : v < (long long) INT32_MIN ? INT32_MIN : (int) v;
+	return __fmul_rn(__int2float_rn(c), 9.5367431640625e-07f);
 }
 
 // x86-64 float -> unsigned conversion (via a truncating 64-bit convert)
@@ -144,19 +146,21 @@ __device__ __forceinline__ bool update_izhikevich(const LibmCalib& calib, Neuron
 	}
 	float u = R.x[0], v = R.x[1];
 	const double dI = (double) I;
+	// a sub-step after the one that fired changes nothing: selected, not
+	// branched around
 	bool fired = false;
 #pragma unroll
 	for(int k = 0; k < 4; ++k) {
-		if(!fired) {
-			double vd = (double) v;
-			double t = __dadd_rn(__dmul_rn(0.04, vd), 5.0);
-			t = __dadd_rn(__dmul_rn(t, vd), 140.0);
-			t = __dsub_rn(t, (double) u);
-			t = __dadd_rn(t, dI);
-			v = __double2float_rn(__dadd_rn(vd, __dmul_rn(0.25, t)));
-			u = __fadd_rn(u, __fmul_rn(0.25f, __fmul_rn(a, __fsub_rn(__fmul_rn(b, v), u))));
-			fired = v >= 30.0f;
-		}
+		double vd = (double) v;
+		double t = __dadd_rn(__dmul_rn(0.04, vd), 5.0);
+		t = __dadd_rn(__dmul_rn(t, vd), 140.0);
+		t = __dsub_rn(t, (double) u);
+		t = __dadd_rn(t, dI);
+		const float v1 = __double2float_rn(__dadd_rn(vd, __dmul_rn(0.25, t)));
+		const float u1 = __fadd_rn(u, __fmul_rn(0.25f, __fmul_rn(a, __fsub_rn(__fmul_rn(b, v1), u))));
+		v = fired ? v : v1;
+		u = fired ? u : u1;
+		fired = fired || v1 >= 30.0f;
 	}
 	fired = fired || fs;
 	if(fired) {

@@ -342,16 +342,15 @@ __device__ __forceinline__ void update_range(const DevSim& S, uint32_t first, ui
 
 // Adds the CTA's counters to those of ring position `ring` and clears them
 // (after a __syncthreads that follows the last update_range of the step).
+// By one thread.
 __device__ __forceinline__ void flush_counters(const DevSim& S, uint32_t ring, CtaCounters& C)
 {
-	if(threadIdx.x == 0) {
-		if(C.fired) atomicAdd(&S.firedCount[ring], C.fired);
-		if(C.events) atomicAdd(&S.eventCount[ring], C.events);
-		if(C.stdp) atomicAdd(&S.stdpCount[ring], C.stdp);
-		C.fired = 0;
-		C.events = 0;
-		C.stdp = 0;
-	}
+	if(C.fired) atomicAdd(&S.firedCount[ring], C.fired);
+	if(C.events) atomicAdd(&S.eventCount[ring], C.events);
+	if(C.stdp) atomicAdd(&S.stdpCount[ring], C.stdp);
+	C.fired = 0;
+	C.events = 0;
+	C.stdp = 0;
 }
 
 // One step's neuron update: CTA c owns the partition of P consecutive
@@ -373,7 +372,7 @@ update_kernel(const DevSim S, uint32_t P, uint32_t cur, uint32_t ring, uint32_t 
 	const uint32_t first = blockIdx.x * P;
 	update_range(S, first, min(S.N, first + P), cur, ring, cycleLo, sC, false, hostFired);
 	__syncthreads();
-	flush_counters(S, ring, sC);
+	if(threadIdx.x == 0) flush_counters(S, ring, sC);
 }
 
 // the update_kernel instance for the two-launch step's threads per CTA
@@ -728,7 +727,7 @@ __device__ __forceinline__ bool persistent_step(const DevSim& S, uint32_t P, uns
 		update_range(S, p * P, min(S.N, p * P + P), cur, ring, (uint32_t) c, sC, true, hostFired);
 	}
 	__syncthreads();
-	flush_counters(S, ring, sC);
+	if(threadIdx.x == 0) flush_counters(S, ring, sC);
 	trace_mark(S, row, 3);
 	const bool ok = grid_barrier(gb, sTarget, sOk, S.waitLimit);
 	trace_mark(S, row, 4);
@@ -921,6 +920,70 @@ __device__ __forceinline__ uint32_t wait_request(GridBarrier* gb, uint32_t want,
 	return sCmd;
 }
 
+// CTA 0 takes request `want` from the host and broadcasts it (the other CTAs
+// finished the last step at its final barrier); every thread of a CTA gets 1,
+// or 0 when the loop ends.
+__device__ __forceinline__ uint32_t take_request(const DevSim& S, GridBarrier* gb, ServeCtl* ctl, uint32_t want,
+		uint32_t ring, unsigned long long idleNs, uint32_t& sOk)
+{
+	__shared__ uint32_t sOp;
+	uint32_t op;
+	if(blockIdx.x == 0) {
+		if(threadIdx.x < 32) {
+			// warp 0 reads the request line -- the two request words and
+			// the inline stimulus -- in one 64-byte read per poll
+			const uint32_t FULL = 0xffffffffu, lane = threadIdx.x;
+			const unsigned long long* line = &ctl->req[0];
+			op = 0;
+			const unsigned long long t0 = global_ns();
+			for(uint32_t polls = 0; polls < SERVE_POLL_LIMIT; ++polls) {
+				const unsigned long long w = lane < 2 + SERVE_INLINE ? ld_relaxed_sys_u64(line + lane) : 0ull;
+				const unsigned long long a = __shfl_sync(FULL, w, 0);
+				const unsigned long long b = __shfl_sync(FULL, w, 1);
+				bool got = (uint32_t) (a >> 32) == want && (uint32_t) (b >> 32) == want;
+				const bool inl = got && ((uint32_t) a & SERVE_INLINE_FLAG) != 0u;
+				const uint32_t count = (uint32_t) a & ~SERVE_INLINE_FLAG;
+				const bool mine = inl && lane >= 2 && lane - 2 < count;
+				if(inl) got = __all_sync(FULL, !mine || (uint32_t) (w >> 32) == want);
+				if(got) {
+					// the stimulus the host wrote before the request
+					asm volatile("fence.acq_rel.sys;" ::: "memory");
+					// an inline firing stimulus is applied here; the step's
+					// first grid barrier orders it before the update reads it
+					if(mine) {
+						const uint32_t l = (uint32_t) w;
+						atomicOr(&S.fstim[l >> 5], 1u << (l & 31));
+					}
+					if(lane == 0) {
+						gb->nf = inl ? 0u : (uint32_t) a;
+						gb->ni = (uint32_t) b;
+						S.eventCount[ring] = 0;
+					}
+					op = 1;
+					break;
+				}
+				uint32_t stop = 0;
+				if(lane == 0) {
+					stop = (uint32_t) (a >> 32) == (want | SERVE_STOP) || global_ns() - t0 > idleNs
+							|| ((polls & 1023u) == 1023u && ld_acquire(&gb->error));
+				}
+				if(__shfl_sync(FULL, stop, 0)) break;
+				__nanosleep(32);
+			}
+			__syncwarp();
+			if(lane == 0) {
+				st_release(&gb->cmd, op ? want : want | SERVE_STOP);
+				sOp = op;
+			}
+		}
+		__syncthreads();
+		op = sOp;
+	} else {
+		op = wait_request(gb, want, sOk, S.waitLimit);
+	}
+	return op;
+}
+
 template<unsigned MAXT, unsigned MINB>
 __global__ void __launch_bounds__(MAXT, MINB)
 serve_kernel(const DevSim S, uint32_t P, unsigned long long cycle0, GridBarrier* gb, ServeCtl* ctl, uint32_t seq0,
@@ -934,67 +997,11 @@ serve_kernel(const DevSim S, uint32_t P, unsigned long long cycle0, GridBarrier*
 		sOk = 1;
 	}
 	__syncthreads();
-	__shared__ uint32_t sOp;
 	uint32_t want = seq0;
 	for(unsigned long long k = 0;; ++k, want = serve_next(want)) {
 		const unsigned long long c = cycle0 + k;
 		const uint32_t ring = (uint32_t) (c % S.R);
-		// CTA 0 takes the request from the host and broadcasts it (the
-		// other CTAs finished the last step at its final barrier)
-		uint32_t op;
-		if(blockIdx.x == 0) {
-			if(threadIdx.x < 32) {
-				// warp 0 reads the request line -- the two request words and
-				// the inline stimulus -- in one 64-byte read per poll
-				const uint32_t FULL = 0xffffffffu, lane = threadIdx.x;
-				const unsigned long long* line = &ctl->req[0];
-				op = 0;
-				const unsigned long long t0 = global_ns();
-				for(uint32_t polls = 0; polls < SERVE_POLL_LIMIT; ++polls) {
-					const unsigned long long w = lane < 2 + SERVE_INLINE ? ld_relaxed_sys_u64(line + lane) : 0ull;
-					const unsigned long long a = __shfl_sync(FULL, w, 0);
-					const unsigned long long b = __shfl_sync(FULL, w, 1);
-					bool got = (uint32_t) (a >> 32) == want && (uint32_t) (b >> 32) == want;
-					const bool inl = got && ((uint32_t) a & SERVE_INLINE_FLAG) != 0u;
-					const uint32_t count = (uint32_t) a & ~SERVE_INLINE_FLAG;
-					const bool mine = inl && lane >= 2 && lane - 2 < count;
-					if(inl) got = __all_sync(FULL, !mine || (uint32_t) (w >> 32) == want);
-					if(got) {
-						// the stimulus the host wrote before the request
-						asm volatile("fence.acq_rel.sys;" ::: "memory");
-						// an inline firing stimulus is applied here; the step's
-						// first grid barrier orders it before the update reads it
-						if(mine) {
-							const uint32_t l = (uint32_t) w;
-							atomicOr(&S.fstim[l >> 5], 1u << (l & 31));
-						}
-						if(lane == 0) {
-							gb->nf = inl ? 0u : (uint32_t) a;
-							gb->ni = (uint32_t) b;
-							S.eventCount[ring] = 0;
-						}
-						op = 1;
-						break;
-					}
-					uint32_t stop = 0;
-					if(lane == 0) {
-						stop = (uint32_t) (a >> 32) == (want | SERVE_STOP) || global_ns() - t0 > idleNs
-								|| ((polls & 1023u) == 1023u && ld_acquire(&gb->error));
-					}
-					if(__shfl_sync(FULL, stop, 0)) break;
-					__nanosleep(32);
-				}
-				__syncwarp();
-				if(lane == 0) {
-					st_release(&gb->cmd, op ? want : want | SERVE_STOP);
-					sOp = op;
-				}
-			}
-			__syncthreads();
-			op = sOp;
-		} else {
-			op = wait_request(gb, want, sOk, S.waitLimit);
-		}
+		const uint32_t op = take_request(S, gb, ctl, want, ring, idleNs, sOk);
 		if(!op) return;
 		const uint32_t nf = *(volatile uint32_t*) &gb->nf;
 		const uint32_t ni = *(volatile uint32_t*) &gb->ni;
@@ -1015,6 +1022,719 @@ serve_kernel(const DevSim S, uint32_t P, unsigned long long cycle0, GridBarrier*
 	}
 }
 
+// ---------------------------------------------------------------------------
+// The single-barrier step loop (local_run_kernel, local_serve_kernel)
+//
+// The persistent loop above balances deliveries and STDP entries over the
+// whole grid: lists published through global memory, two grid barriers a
+// step, and chains of dependent loads on either side.  That pays where single
+// groups are long (1000 synapses of one delay).  Where they are short, a step
+// is those chains and barriers: 8.9 us at 1000 neurons x 100 synapses, 11.7 us
+// at 100k x 100.  This loop gives them up:
+//  - a worker thread owns one neuron for the whole launch, its parameters,
+//    state, RNG words and delay-group ends in shared memory and its history
+//    in registers;
+//  - after its update a warp delivers its own neurons' groups for the next
+//    step, flattened from a list in its own shared memory, four synapses a
+//    lane per round, and accumulates STDP for its own neurons that are targets;
+//  - a step has one barrier, between the deliveries to it and its update.  A
+//    CTA that has passed it may deliver to the next step while others still
+//    read this one's sums: the accumulators alternate between two buffers.
+//    The STDP accumulation of step t runs while the barrier of t + 1
+//    completes; with delays of at least 1 it needs its sources' histories of
+//    step t - 1 only, which rotate over three buffers;
+//  - the last warp signals and awaits the barrier, and some warps before it
+//    draw the noise of the coming step all along (local_noise): on the worker
+//    warps the draw, and on the first of them the wait for its own arrival
+//    too, lay on the step's path (100k x 100: 8.8 us a step; reading the
+//    draws from the libm tables a step ahead instead: 10.0).
+// What stays in memory between launches is what the other loops keep, except
+// the work lists, which publish_kernel rebuilds from the histories when
+// another loop follows (Simulation::ensureLists).
+//
+// SYNC: how the CTAs wait for one another, and where the accumulators are.
+// 1: one cluster, an mbarrier in each CTA's shared memory at which every CTA's
+// arrival is signalled; the accumulators lie in the owner's shared memory, as
+// four 32-bit words: a weight w adds its low 16 bits to one word and w >> 16
+// to another (no carry to pass on, exact for up to 65536 arrivals a step).
+// 2: the grid barrier above, accumulators in global memory as in the other
+// loops.  planLocal says which is taken when.
+constexpr uint32_t LOCAL_GROUPS = 128;  // groups of a warp's list at a time
+constexpr uint32_t LOCAL_ACC = 8;       // accumulator words of a neuron in shared memory: two buffers of four
+constexpr uint32_t LOCAL_THREADS = 1024;
+constexpr size_t LOCAL_SMEM_MAX = 200 * 1024;  // the resident form has 17 KB of its own
+constexpr uint32_t LOCAL_WORDS = 15;    // words of a neuron: at most 13 of parameters, state and RNG
+constexpr uint32_t LOCAL_NOISE = 11;    // an Izhikevich neuron's noise by step parity, then the RNG words its last draw shifted out
+constexpr uint32_t LOCAL_BAR = 2;       // named barrier of the workers and the last warp
+
+template<int SYNC>
+struct LoopBarrier {
+	GridBarrier* gb;
+	uint32_t* target;            // SYNC 2 (shared)
+	uint32_t* ok;                // (shared)
+	unsigned long long* mbar;    // SYNC 1 (shared)
+	uint32_t limit;
+	uint32_t phase = 0;
+
+	__device__ __forceinline__ LoopBarrier(GridBarrier* g, uint32_t* t, uint32_t* o, unsigned long long* m, uint32_t lim,
+			uint32_t base) : gb(g), target(t), ok(o), mbar(m), limit(lim)
+	{
+		if(threadIdx.x == 0) {
+			*target = base;
+			*ok = 1;
+			if(SYNC == 1) {
+				const uint32_t a = (uint32_t) __cvta_generic_to_shared(mbar);
+				asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(a), "r"(gridDim.x) : "memory");
+				asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+			}
+		}
+		if(SYNC == 1) cluster_sync();
+		else __syncthreads();
+	}
+
+	// every CTA is in the cluster barrier once at its start and once at its
+	// end: no arrival meets a CTA that has not begun or has left
+	__device__ __forceinline__ void cluster_sync()
+	{
+		asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+		asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+	}
+
+	__device__ __forceinline__ void finish()
+	{
+		if(SYNC == 1) {
+			__syncthreads();
+			cluster_sync();
+		}
+	}
+
+	// The last warp, after the workers of its CTA: the CTA arrives, `after`
+	// runs on one lane, and the warp waits for the other CTAs.
+	template<typename F>
+	__device__ __forceinline__ void arrive_and_wait(F after)
+	{
+		const uint32_t lane = threadIdx.x & 31;
+		if constexpr(SYNC == 2) {
+			if(lane == 0) {
+				const uint32_t t = *target + gridDim.x;
+				*target = t;
+				red_release_add(&gb->count, 1u);
+				after();
+				for(uint32_t polls = 0; !reached(ld_acquire(&gb->count), t);) {
+					if(give_up(gb, polls, limit)) {
+						fail();
+						break;
+					}
+				}
+			}
+		} else {
+			__syncwarp();
+			const uint32_t a = (uint32_t) __cvta_generic_to_shared(mbar);
+			if(lane < gridDim.x) {
+				asm volatile("{\n\t.reg .b32 r;\n\tmapa.shared::cluster.u32 r, %0, %1;\n\t"
+						"mbarrier.arrive.release.cluster.shared::cluster.b64 _, [r];\n\t}" :: "r"(a), "r"(lane) : "memory");
+			}
+			if(lane == 0) {
+				after();
+				for(uint32_t polls = 0;;) {
+					uint32_t done;
+					asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+							"selp.b32 %0, 1, 0, p;\n\t}" : "=r"(done) : "r"(a), "r"(phase & 1u) : "memory");
+					if(done) break;
+					if(give_up(gb, polls, limit)) {
+						fail();
+						break;
+					}
+				}
+			}
+			++phase;
+		}
+	}
+
+	__device__ __forceinline__ void fail()
+	{
+		atomicExch(&gb->error, 1u);
+		*ok = 0;
+	}
+
+	// joins the CTA's threads after arrive_and_wait
+	__device__ __forceinline__ bool join()
+	{
+		__syncthreads();
+		return *ok != 0;
+	}
+};
+
+// the CTA barrier of the workers and the last warp (the noise warps run on)
+__device__ __forceinline__ void local_workers_sync(uint32_t workers)
+{
+	asm volatile("bar.sync %0, %1;" :: "n"(LOCAL_BAR), "r"(workers + 32) : "memory");
+}
+
+// a CTA's counts of one step: sums over distinct neurons, so they fit 32 bits
+// (a network has fewer than 2^32 synapses)
+struct LocalCounters {
+	uint32_t fired, events, stdp;
+};
+
+__device__ __forceinline__ void flush_counters(const DevSim& S, uint32_t ring, LocalCounters& C)
+{
+	const LocalCounters c = C;
+	if(c.fired) atomicAdd(&S.firedCount[ring], c.fired);
+	if(c.events) atomicAdd(&S.eventCount[ring], (unsigned long long) c.events);
+	if(c.stdp) atomicAdd(&S.stdpCount[ring], (unsigned long long) c.stdp);
+	C = LocalCounters{ 0, 0, 0 };
+}
+
+// one neuron's words in shared memory: word k of thread t at words[k * T + t]
+__device__ __forceinline__ void local_load(const uint32_t* words, uint32_t T, int kind, NeuronRegs& R)
+{
+	auto f = [&](uint32_t k) { return __uint_as_float(words[k * T]); };
+	switch(kind) {
+		case KIND_IZHIKEVICH:
+#pragma unroll
+			for(int k = 0; k < 5; ++k) R.p[k] = f(k);
+			R.x[0] = f(5);
+			R.x[1] = f(6);
+			break;
+		case KIND_IF_CURR_EXP:
+#pragma unroll
+			for(int k = 0; k < 9; ++k) R.p[k] = f(k);
+#pragma unroll
+			for(int k = 0; k < 4; ++k) R.x[k] = f(9 + k);
+			break;
+		case KIND_POISSON:
+			R.p[0] = f(0);
+#pragma unroll
+			for(int k = 0; k < 4; ++k) R.r[k] = words[(1 + k) * T];
+			break;
+		case KIND_IZHIKEVICH_RS:
+			R.x[0] = f(0);
+			R.x[1] = f(1);
+			break;
+		default:
+			break;
+	}
+}
+
+__device__ __forceinline__ void local_store(uint32_t* words, uint32_t T, int kind, const NeuronRegs& R)
+{
+	switch(kind) {
+		case KIND_IZHIKEVICH:
+			words[5 * T] = __float_as_uint(R.x[0]);
+			words[6 * T] = __float_as_uint(R.x[1]);
+			break;
+		case KIND_IF_CURR_EXP:
+#pragma unroll
+			for(int k = 0; k < 4; ++k) words[(9 + k) * T] = __float_as_uint(R.x[k]);
+			break;
+		case KIND_POISSON:
+#pragma unroll
+			for(int k = 0; k < 4; ++k) words[(1 + k) * T] = R.r[k];
+			break;
+		case KIND_IZHIKEVICH_RS:
+			words[0] = __float_as_uint(R.x[0]);
+			words[T] = __float_as_uint(R.x[1]);
+			break;
+		default:
+			break;
+	}
+}
+
+// the neuron of this worker thread for a launch
+struct LocalNeuron {
+	uint32_t n, nl, T;
+	int kind;                // -1: none
+	const TypeRange* type;
+	uint32_t* words;         // its column of the shared words [LOCAL_WORDS][T]
+	const uint16_t* ends;    // its row of delay-group ends (shared)
+	uint32_t* list;          // its warp's list (shared)
+	uint32_t* acc;           // SYNC 1: the CTA's accumulators [2][4][T] (shared)
+	uint64_t h, dm;          // history, delays it has synapses of
+	uint32_t ob, outdeg, rb, indeg;
+};
+
+// The neuron of worker i: the words of 32 neurons go round the CTAs, so that
+// neurons of a kind (the inhibitory fifth, a busy type) spread over all of
+// them.
+__device__ __forceinline__ uint32_t local_index(uint32_t i)
+{
+	return ((i >> 5) * gridDim.x + blockIdx.x) * 32 + (i & 31);
+}
+
+__device__ __forceinline__ const TypeRange& local_type(const DevSim& S, uint32_t n)
+{
+	uint32_t k = 0;
+	while(k + 1 < S.ntypes && n >= S.types[k + 1].base) ++k;
+	return S.types[k];
+}
+
+// parameters, state and RNG words that a neuron of a kind keeps in its column
+__device__ __forceinline__ void local_layout(int kind, uint32_t& np, uint32_t& ns, uint32_t& nr)
+{
+	np = ns = nr = 0;
+	switch(kind) {
+		case KIND_IZHIKEVICH: np = 5; ns = 2; nr = 4; break;
+		case KIND_IF_CURR_EXP: np = 9; ns = 4; break;
+		case KIND_POISSON: np = 1; nr = 4; break;
+		case KIND_IZHIKEVICH_RS: ns = 2; break;
+		default: break;
+	}
+}
+
+template<int SYNC>
+__device__ __forceinline__ void local_begin(const DevSim& S, const LocalLoop& A, unsigned char* raw, LocalNeuron& L)
+{
+	const uint32_t T = A.workers, tid = threadIdx.x;
+	uint32_t* words = reinterpret_cast<uint32_t*>(raw);
+	uint32_t* lists = words + LOCAL_WORDS * T;
+	L.acc = lists + (T >> 5) * 2 * LOCAL_GROUPS;
+	uint16_t* ends = reinterpret_cast<uint16_t*>(L.acc + (SYNC == 2 ? 0 : LOCAL_ACC * T));
+	L.list = lists + (tid >> 5) * 2 * LOCAL_GROUPS;
+	L.T = T;
+	L.n = local_index(tid);
+	L.words = words + tid;
+	L.ends = ends + (size_t) tid * A.rowStride;
+	L.kind = -1;
+	L.type = &S.types[0];
+	L.h = L.dm = 0;
+	L.ob = L.outdeg = L.rb = L.indeg = 0;
+	L.nl = 0;
+	for(uint32_t w = tid >> 5; w < T >> 5; w += blockDim.x >> 5) {
+		// the rows of a word's neurons are contiguous
+		const uint32_t first = local_index(w * 32);
+		if(first >= S.N) break;
+		for(uint32_t i = tid & 31; i < min(32u, S.N - first) * S.dStride; i += 32) {
+			const uint32_t r = i / S.dStride;
+			ends[(size_t) (w * 32 + r) * A.rowStride + (i - r * S.dStride)] = S.dEnd16[(size_t) first * S.dStride + i];
+		}
+	}
+	if(SYNC != 2) {
+		for(uint32_t k = tid; k < LOCAL_ACC * T; k += blockDim.x) L.acc[k] = 0;
+	}
+	if(tid < T && L.n < S.N) {
+		L.type = &local_type(S, L.n);
+		L.kind = L.type->kind;
+		L.nl = L.n - L.type->base;
+		const uint32_t n = L.n;
+		L.h = S.hist[(size_t) ((A.cycle0 & 1) ^ 1) * S.N + n];
+		L.dm = S.delayMask[n];
+		L.ob = (uint32_t) S.outPtr[n];
+		L.outdeg = (uint32_t) (S.outPtr[n + 1] - S.outPtr[n]);
+		if(S.stdp) {
+			L.rb = (uint32_t) S.rcmPtr[n];
+			L.indeg = (uint32_t) (S.rcmPtr[n + 1] - S.rcmPtr[n]);
+			S.hist3[(size_t) ((A.cycle0 + 2) % 3) * S.N + n] = L.h;
+		}
+		const uint32_t nn = L.type->n, nl = L.nl;
+		uint32_t np, ns, nr;
+		local_layout(L.kind, np, ns, nr);
+		for(uint32_t j = 0; j < np; ++j) L.words[j * T] = __float_as_uint(L.type->param[j * nn + nl]);
+		for(uint32_t j = 0; j < ns; ++j) L.words[(np + j) * T] = __float_as_uint(L.type->state[j * nn + nl]);
+		for(uint32_t j = 0; j < nr; ++j) L.words[(np + ns + j) * T] = S.rng[j * S.N + n];
+	}
+}
+
+// Writes back what a launch changed; `last` = the parity of its last step.
+// ahead: a noise draw that no step used is undone.
+__device__ __forceinline__ void local_end(const DevSim& S, const LocalNeuron& L, uint32_t last, bool ahead)
+{
+	if(L.kind < 0) return;
+	const uint32_t T = L.T, nn = L.type->n, nl = L.nl;
+	uint32_t np, ns, nr;
+	local_layout(L.kind, np, ns, nr);
+	for(uint32_t j = 0; j < ns; ++j) L.type->state[j * nn + nl] = __uint_as_float(L.words[(np + j) * T]);
+	if(ahead && L.kind == KIND_IZHIKEVICH && __uint_as_float(L.words[4 * T]) != 0.0f) {
+		// a draw shifts two words out and two in
+		S.rng[L.n] = L.words[(LOCAL_NOISE + 2) * T];
+		S.rng[S.N + L.n] = L.words[(LOCAL_NOISE + 3) * T];
+		S.rng[2 * S.N + L.n] = L.words[7 * T];
+		S.rng[3 * S.N + L.n] = L.words[8 * T];
+	} else {
+		for(uint32_t j = 0; j < nr; ++j) S.rng[j * S.N + L.n] = L.words[(np + ns + j) * T];
+	}
+	S.hist[(size_t) last * S.N + L.n] = L.h;
+}
+
+// The noise warps (threads [T, blockDim.x - 32)): the nrand of the coming step
+// (parity cur) of the CTA's Izhikevich neurons, each thread several in turn.
+// It depends on their RNG words only, which nobody else touches.
+__device__ __forceinline__ void local_noise(const DevSim& S, unsigned char* raw, uint32_t T, uint32_t cur)
+{
+	uint32_t* words = reinterpret_cast<uint32_t*>(raw);
+	for(uint32_t i = threadIdx.x - T; i < T; i += blockDim.x - 32 - T) {
+		uint32_t* w = words + i;
+		const uint32_t n = local_index(i);
+		if(n >= S.N || local_type(S, n).kind != KIND_IZHIKEVICH || __uint_as_float(w[4 * T]) == 0.0f) continue;
+		uint32_t r[4];
+#pragma unroll
+		for(uint32_t k = 0; k < 4; ++k) r[k] = w[(7 + k) * T];
+		w[(LOCAL_NOISE + 2) * T] = r[0];
+		w[(LOCAL_NOISE + 3) * T] = r[1];
+		w[(LOCAL_NOISE + cur) * T] = __float_as_uint(nb_nrand<true>(S.calib, r[0], r[1], r[2], r[3]));
+#pragma unroll
+		for(uint32_t k = 0; k < 4; ++k) w[(7 + k) * T] = r[k];
+	}
+}
+
+// Adds synapse {tg, w} to its target's accumulator in buffer `buf`.
+// rankMul divides a word index by the number of CTAs (local_index).
+template<int SYNC>
+__device__ __forceinline__ void local_add(const DevSim& S, const LocalNeuron& L, uint32_t buf, uint32_t rankMul, uint32_t tg,
+		int32_t w)
+{
+	const uint32_t t = tg & (MAX_NEURONS - 1);
+	if(SYNC == 2) {
+		unsigned long long* a = reinterpret_cast<unsigned long long*>(S.slot2 + (size_t) buf * S.N + t);
+		red_add_u64(a + (w >= 0 ? 0 : 1), (unsigned long long) (long long) w);
+	} else {
+		const uint32_t word = t >> 5, row = __umulhi(word, rankMul), rank = word - row * gridDim.x;
+		uint32_t a = (uint32_t) __cvta_generic_to_shared(L.acc + (buf * 4 + (w >= 0 ? 0 : 2)) * L.T + row * 32 + (t & 31));
+		const uint32_t lo = (uint32_t) w & 0xffffu;
+		const int32_t hi = w >> 16;
+		asm volatile("mapa.shared::cluster.u32 %0, %0, %1;" : "+r"(a) : "r"(rank));
+		asm volatile("red.relaxed.cluster.shared::cluster.add.u32 [%0], %1;" :: "r"(a), "r"(lo) : "memory");
+		if(hi) asm volatile("red.relaxed.cluster.shared::cluster.add.s32 [%0], %1;" :: "r"(a + 4 * L.T), "r"(hi) : "memory");
+	}
+}
+
+// the forward matrix is constant during a launch; a small network's rows
+// stay in L1
+template<int SYNC>
+__device__ __forceinline__ uint32_t local_synapse(const uint32_t* p)
+{
+	return SYNC == 2 ? __ldcs(p) : __ldg(p);
+}
+
+// Delivers the groups `pend` (bit d - 1: delay d) of the warp's neurons into
+// buffer `buf`, as process_list<0>.
+template<int SYNC>
+__device__ __forceinline__ void local_deliver(const DevSim& S, const LocalNeuron& L, uint32_t buf, uint32_t rankMul, uint64_t pend)
+{
+	const uint32_t FULL = 0xffffffffu, lane = threadIdx.x & 31;
+	uint32_t* start = L.list;
+	uint32_t* offset = L.list + LOCAL_GROUPS;
+	const uint32_t below = (1u << lane) - 1u;
+	while(__any_sync(FULL, pend != 0)) {
+		constexpr uint32_t PER = LOCAL_GROUPS / 32;  // groups of a lane per pass
+		uint32_t st[PER], len[PER], ng = 0, ne = 0;
+#pragma unroll
+		for(uint32_t j = 0; j < PER; ++j) {
+			st[j] = len[j] = 0;
+			if(pend) {
+				const uint32_t d = (uint32_t) __ffsll((long long) pend);
+				pend &= pend - 1;
+				const uint32_t e0 = d > 1 ? L.ends[d - 2] : 0u, e1 = L.ends[d - 1];
+				st[j] = L.ob + e0;
+				len[j] = e1 - e0;
+				ne += len[j];
+				++ng;
+			}
+		}
+		// prefix sums of the groups (0 to 4 a lane: by ballots of the bits) and
+		// of the entries
+		const uint32_t g0 = __ballot_sync(FULL, ng & 1u), g1 = __ballot_sync(FULL, ng & 2u), g2 = __ballot_sync(FULL, ng & 4u);
+		const uint32_t groups = __popc(g0) + 2 * __popc(g1) + 4 * __popc(g2);
+		uint32_t g = __popc(g0 & below) + 2 * __popc(g1 & below) + 4 * __popc(g2 & below);
+		const uint32_t ie = warp_inclusive_scan(ne);
+		const uint32_t total = __shfl_sync(FULL, ie, 31);
+		uint32_t e = ie - ne;
+#pragma unroll
+		for(uint32_t j = 0; j < PER; ++j) {
+			if(j < ng) {
+				start[g + j] = st[j];
+				offset[g + j] = e;
+				e += len[j];
+			}
+		}
+		__syncwarp();
+		const uint32_t top = groups > 1 ? 1u << (31 - __clz(groups - 1)) : 0u;
+		for(uint32_t base = 0; base < total; base += 128) {
+			// the last group that starts at or before each entry
+			uint32_t q[4] = { 0, 0, 0, 0 };
+			const uint32_t left = total - base;
+			for(uint32_t step = top; step; step >>= 1) {
+#pragma unroll
+				for(uint32_t j = 0; j < 4; ++j) {
+					if(32 * j < left && q[j] + step < groups && offset[q[j] + step] <= base + lane + 32 * j) q[j] += step;
+				}
+			}
+			uint32_t tg[4];
+			int32_t w[4];
+#pragma unroll
+			for(uint32_t j = 0; j < 4; ++j) {
+				const uint32_t x = base + lane + 32 * j;
+				if(x < total) {
+					const uint32_t i = start[q[j]] + (x - offset[q[j]]);
+					tg[j] = local_synapse<SYNC>(S.synTgt + i);
+					w[j] = (int32_t) local_synapse<SYNC>(S.synW + i);
+				}
+			}
+#pragma unroll
+			for(uint32_t j = 0; j < 4; ++j) {
+				if(base + lane + 32 * j < total) local_add<SYNC>(S, L, buf, rankMul, tg[j], w[j]);
+			}
+		}
+		__syncwarp();
+	}
+}
+
+// STDP accumulation of this step over the incoming plastic synapses of the
+// warp's targets, as process_list<1>, with the histories `prev` of the step
+// before: shifted by one, they are this step's but for the newest bit, which
+// a delay of at least 1 shifts out
+__device__ __forceinline__ void local_stdp(const DevSim& S, const LocalNeuron& L, bool target, const uint64_t* prev)
+{
+	const uint32_t FULL = 0xffffffffu, lane = threadIdx.x & 31;
+	if(!__any_sync(FULL, target)) return;
+	const uint32_t len = target ? L.indeg : 0u;
+	const uint32_t incl = warp_inclusive_scan(len);
+	const uint32_t total = __shfl_sync(FULL, incl, 31);
+	for(uint32_t base = 0; base < total; base += 128) {
+		uint32_t idx[4], sd[4];
+		uint64_t h[4];
+#pragma unroll
+		for(uint32_t j = 0; j < 4; ++j) {
+			const uint32_t x = base + lane + 32 * j;
+			uint32_t r = 0;
+#pragma unroll
+			for(uint32_t step = 16; step; step >>= 1) {
+				if(__shfl_sync(FULL, incl, r + step - 1) <= x) r += step;
+			}
+			idx[j] = __shfl_sync(FULL, L.rb, r) + (x - __shfl_sync(FULL, incl - len, r));
+			sd[j] = x < total ? __ldcs(S.rcmSrc + idx[j]) : 0u;
+		}
+#pragma unroll
+		for(uint32_t j = 0; j < 4; ++j) {
+			h[j] = base + lane + 32 * j < total ? __ldcg(prev + (sd[j] & (MAX_NEURONS - 1))) : 0ull;
+		}
+#pragma unroll
+		for(uint32_t j = 0; j < 4; ++j) {
+			if(base + lane + 32 * j < total) {
+				const uint32_t delay = (sd[j] >> 26) + 1;
+				const int32_t dw = stdp_weight_change(S.sp, (h[j] << 1) >> delay);
+				if(dw != 0) red_add_s32(S.rcmAcc + idx[j], dw);
+			}
+		}
+	}
+}
+
+// Update of step c (cur = c & 1, ring row ring) for this thread's neuron;
+// returns whether it is an STDP target of this step
+template<int SYNC, bool STIM>
+__device__ __forceinline__ bool local_update(const DevSim& S, LocalNeuron& L, unsigned long long c, uint32_t ring, LocalCounters& C)
+{
+	const uint32_t lane = threadIdx.x & 31, buf = (uint32_t) (c & 1);
+	bool fired = false, target = false;
+	uint32_t fw = 0;
+	if(L.kind >= 0) {
+		long long sumE, sumI;
+		if(SYNC == 2) {
+			ulonglong2* slot = S.slot2 + (size_t) buf * S.N + L.n;
+			const ulonglong2 acc = __ldcg(slot);
+			if(acc.x | acc.y) *slot = make_ulonglong2(0, 0);
+			sumE = (long long) acc.x;
+			sumI = (long long) acc.y;
+		} else {
+			uint32_t* a = L.acc + buf * 4 * L.T + threadIdx.x;
+			sumE = (long long) (int32_t) a[L.T] * 65536 + a[0];
+			sumI = (long long) (int32_t) a[3 * L.T] * 65536 + a[2 * L.T];
+#pragma unroll
+			for(uint32_t k = 0; k < 4; ++k) a[k * L.T] = 0;
+		}
+		float ext = 0.0f;
+		if(STIM) {
+			ext = __ldcg(S.curExt + L.n);
+			fw = __ldcg(S.fstim + (L.n >> 5));
+		}
+		NeuronRegs R;
+		local_load(L.words, L.T, L.kind, R);
+		R.pre = true;
+		R.noise = L.kind == KIND_IZHIKEVICH ? __uint_as_float(L.words[(LOCAL_NOISE + buf) * L.T]) : 0.0f;
+		if(STIM && __float_as_uint(ext) != 0u) S.curExt[L.n] = 0.0f;
+		const float cE = wfx_to_float(sumE);
+		const float cI = wfx_to_float(sumI);
+		TypeRange t;
+		t.kind = L.kind;
+		fired = update_neuron(S, t, R, cE, cI, ext, (fw >> lane) & 1u);
+		local_store(L.words, L.T, L.kind, R);
+		L.h = (L.h << 1) | (uint64_t) fired;
+		if(S.stdp) {
+			S.hist3[(size_t) (c % 3) * S.N + L.n] = L.h;
+			target = (L.h & S.sp.postFireMask) && L.indeg > 0;
+		}
+	}
+	const uint32_t fb = __ballot_sync(0xffffffffu, fired);
+	if(lane == 0 && L.kind >= 0) {
+		S.firedRing[(size_t) ring * S.W + (L.n >> 5)] = fb;
+		if(STIM && fw) S.fstim[L.n >> 5] = 0u;
+	}
+	if(fb) {
+		const uint32_t ev = __reduce_add_sync(0xffffffffu, fired ? L.outdeg : 0u);
+		if(lane == 0) {
+			atomicAdd(&C.fired, (uint32_t) __popc(fb));
+			atomicAdd(&C.events, ev);
+		}
+	}
+	const uint32_t tb = __ballot_sync(0xffffffffu, target);
+	if(tb) {
+		const uint32_t se = __reduce_add_sync(0xffffffffu, target ? L.indeg : 0u);
+		if(lane == 0) {
+			atomicOr(&S.touchedBits[L.n >> 5], tb);
+			atomicAdd(&C.stdp, se);
+		}
+	}
+	return target;
+}
+
+// `steps` steps from cycle0, as run_kernel; the last step's deliveries stay
+// pending (the next launch, or publish_kernel, finds them in the histories).
+template<int SYNC>
+__global__ void __launch_bounds__(LOCAL_THREADS, 1)
+local_run_kernel(const DevSim S, const LocalLoop A)
+{
+	extern __shared__ __align__(16) unsigned char raw[];
+	__shared__ LocalCounters sC[2];  // by step parity: one is emptied while the other fills
+	__shared__ uint32_t sTarget, sOk;
+	__shared__ unsigned long long sBar;
+	LocalNeuron L;
+	local_begin<SYNC>(S, A, raw, L);
+	if(threadIdx.x < 2) sC[threadIdx.x] = LocalCounters{ 0, 0, 0 };
+	LoopBarrier<SYNC> bar(A.gb, &sTarget, &sOk, &sBar, S.waitLimit, A.base);
+	const bool worker = threadIdx.x < A.workers, last = threadIdx.x >= blockDim.x - 32;
+	bool target = false;
+	for(uint32_t k = 0; k < A.steps; ++k) {
+		const unsigned long long c = A.cycle0 + k;
+		const uint32_t cur = (uint32_t) (c & 1);
+		if(worker) {
+			local_deliver<SYNC>(S, L, cur, A.rankMul, L.h & L.dm);
+			local_workers_sync(A.workers);
+			if(S.stdp && k) local_stdp(S, L, target, S.hist3 + (size_t) ((c + 1) % 3) * S.N);
+		} else if(last) {
+			local_workers_sync(A.workers);
+			bar.arrive_and_wait([&] { if(k) flush_counters(S, (uint32_t) ((c - 1) % S.R), sC[cur ^ 1]); });
+		} else {
+			local_noise(S, raw, A.workers, cur);
+		}
+		if(!bar.join()) {
+			bar.finish();
+			return;
+		}
+		if(worker) target = local_update<SYNC, false>(S, L, c, (uint32_t) (c % S.R), sC[cur]);
+	}
+	const unsigned long long end = A.cycle0 + A.steps;
+	if(worker) {
+		if(S.stdp) local_stdp(S, L, target, S.hist3 + (size_t) ((end + 1) % 3) * S.N);
+		local_end(S, L, (uint32_t) ((end - 1) & 1), false);
+	}
+	__syncthreads();
+	if(threadIdx.x == 0) flush_counters(S, (uint32_t) ((end - 1) % S.R), sC[(end - 1) & 1]);
+	bar.finish();
+}
+
+// The resident loop of nemo_step over the same step (serve_kernel): a request
+// starts with its deliveries; the STDP accumulation follows the answer, and
+// the noise is drawn while the loop waits for the request.
+template<int SYNC>
+__global__ void __launch_bounds__(LOCAL_THREADS, 1)
+local_serve_kernel(const DevSim S, const LocalLoop A, ServeCtl* ctl, uint32_t seq0, const uint32_t* stim,
+		uint32_t* hostIds, unsigned long long idleNs)
+{
+	extern __shared__ __align__(16) unsigned char raw[];
+	__shared__ LocalCounters sC;
+	__shared__ uint32_t sTarget, sOk;
+	__shared__ unsigned long long sBar;
+	LocalNeuron L;
+	local_begin<SYNC>(S, A, raw, L);
+	if(threadIdx.x == 0) sC = LocalCounters{ 0, 0, 0 };
+	LoopBarrier<SYNC> bar(A.gb, &sTarget, &sOk, &sBar, S.waitLimit, 0);
+	const bool worker = threadIdx.x < A.workers, last = threadIdx.x >= blockDim.x - 32;
+	uint32_t want = seq0;
+	unsigned long long c = A.cycle0;
+	bool target = false;
+	for(;; ++c, want = serve_next(want)) {
+		const uint32_t cur = (uint32_t) (c & 1), ring = (uint32_t) (c % S.R);
+		if(!worker && !last) local_noise(S, raw, A.workers, cur);
+		if(worker && S.stdp && c > A.cycle0) local_stdp(S, L, target, S.hist3 + (size_t) ((c + 1) % 3) * S.N);
+		if(!take_request(S, A.gb, ctl, want, ring, idleNs, sOk)) break;
+		const uint32_t nf = *(volatile uint32_t*) &A.gb->nf;
+		const uint32_t ni = *(volatile uint32_t*) &A.gb->ni;
+		if(nf + ni) apply_stimulus(S, stim, nf, ni);
+		if(worker) local_deliver<SYNC>(S, L, cur, A.rankMul, L.h & L.dm);
+		__syncthreads();
+		if(last) bar.arrive_and_wait([] {});
+		if(!bar.join()) break;
+		if(worker) target = local_update<SYNC, true>(S, L, c, ring, sC);
+		__syncthreads();
+		if(last) {
+			if((threadIdx.x & 31) == 0) flush_counters(S, ring, sC);
+			__syncwarp();
+			bar.arrive_and_wait([] {});
+		}
+		if(!bar.join()) break;
+		if(blockIdx.x == 0) {
+			const uint32_t n = fired_ids_to_host(S, S.firedRing + (size_t) ring * S.W, hostIds);
+			__syncthreads();
+			if(threadIdx.x == 0) {
+				ctl->fired = n;
+				ctl->events = *(volatile unsigned long long*) &S.eventCount[ring];
+				st_release_sys(&ctl->done, want);
+			}
+		}
+	}
+	__syncthreads();
+	if(worker) local_end(S, L, (uint32_t) ((c - 1) & 1), true);
+	bar.finish();
+}
+
+__global__ void in_degree_kernel(const uint32_t* synTgt, size_t n, uint32_t* count)
+{
+	for(size_t i = (size_t) blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t) gridDim.x * blockDim.x) {
+		atomicAdd(&count[synTgt[i] & (MAX_NEURONS - 1)], 1u);
+	}
+}
+
+// the largest of n values (one block)
+__global__ void max_kernel(const uint32_t* v, uint32_t n, uint32_t* most)
+{
+	uint32_t m = 0;
+	for(uint32_t i = threadIdx.x; i < n; i += blockDim.x) m = max(m, v[i]);
+	m = __reduce_max_sync(0xffffffffu, m);
+	if((threadIdx.x & 31) == 0) atomicMax(most, m);
+}
+
+// The work lists, STDP filter words and counts that the other loops expect
+// after the step of parity `cur`, from the histories (the counts zeroed
+// before).
+__global__ void publish_kernel(const DevSim S, uint32_t cur)
+{
+	const uint32_t lane = threadIdx.x & 31;
+	for(uint32_t base = (blockIdx.x * blockDim.x + threadIdx.x) & ~31u; base < S.N; base += gridDim.x * blockDim.x) {
+		const uint32_t n = base + lane;
+		const uint64_t h = n < S.N ? S.hist[(size_t) cur * S.N + n] : 0ull;
+		const uint64_t pend = n < S.N ? h & S.delayMask[n] : 0ull;
+		const uint32_t rbits = __ballot_sync(0xffffffffu, h != 0);
+		if(lane == 0) S.recent[(size_t) cur * S.recentWords + (n >> 5)] = rbits;
+		uint32_t ng = 0, ne = 0;
+		for(uint64_t b = pend; b; b &= b - 1) {
+			const uint32_t d = (uint32_t) __ffsll((long long) b);
+			ne += delay_end(S, n, d) - delay_end(S, n, d - 1);
+			++ng;
+		}
+		const uint32_t ig = warp_inclusive_scan(ng), ie = warp_inclusive_scan(ne);
+		unsigned long long at = 0;
+		if(lane == 31 && ig) at = atomicAdd(&S.dlvWork.count[cur], ((unsigned long long) ig << 32) | ie);
+		at = __shfl_sync(0xffffffffu, at, 31);
+		uint32_t g = (uint32_t) (at >> 32) + ig - ng, e = (uint32_t) at + ie - ne;
+		for(uint64_t b = pend; b; b &= b - 1) {
+			const uint32_t d = (uint32_t) __ffsll((long long) b);
+			const uint32_t e0 = delay_end(S, n, d - 1), e1 = delay_end(S, n, d);
+			write_group(S.dlvWork, g++, e, S.outPtr[n] + e0, e1 - e0);
+			e += e1 - e0;
+		}
+	}
+}
+
 // The instances of the persistent loops for a block size
 constexpr uint32_t RUN_THREADS_PAIR = 512;
 static const void* run_kernel_for(uint32_t threads, bool trace)
@@ -1023,6 +1743,11 @@ static const void* run_kernel_for(uint32_t threads, bool trace)
 		return trace ? (const void*) run_kernel<true, RUN_THREADS_PAIR, 2> : (const void*) run_kernel<false, RUN_THREADS_PAIR, 2>;
 	}
 	return trace ? (const void*) run_kernel<true, RUN_THREADS, 1> : (const void*) run_kernel<false, RUN_THREADS, 1>;
+}
+static const void* local_kernel_for(int sync, bool serve)
+{
+	if(sync == 1) return serve ? (const void*) local_serve_kernel<1> : (const void*) local_run_kernel<1>;
+	return serve ? (const void*) local_serve_kernel<2> : (const void*) local_run_kernel<2>;
 }
 static const void* serve_kernel_for(uint32_t threads)
 {
@@ -2092,6 +2817,7 @@ void Simulation::init(const std::vector<const Network*>& nets, const Configurati
 		// thread would update more than two neurons in turn, the update is
 		// faster as one launch over the whole network (a large batch)
 		if((uint64_t) N > 2ull * m_runGrid * m_runT) usePersistent = false;
+		if(m_runGrid) planLocal();
 	}
 	NB_CUDA(cudaStreamSynchronize(m_stream));
 	resetTimer();
@@ -2194,10 +2920,174 @@ unsigned Simulation::runGridFor(uint32_t T) const
 	return perSm > 0 ? (unsigned) perSm * (unsigned) m_sms : 0u;
 }
 
+// Whether the single-barrier loop runs this network, and its shape.  A neuron's
+// deliveries and STDP entries are one warp's work there, so it loses where one
+// neuron can bring many.  Microseconds a step, this loop / the persistent one
+// (example networks, 200 steps):
+//   fan-out 100:  1k 3.2 / 8.4,  10k with STDP 5.1 / 10.5,  50k 4.9 / 10.1,  100k 6.0 / 11.2
+//   fan-out 300:  3k 4.5 / 8.4,  20k 6.1 / 9.4,  100k 9.9 / 11.5;
+//                 with STDP 3k 7.2 / 10.0,  20k 10.5 / 11.5,  100k 15.3 / 14.7
+//   fan-out 800 to 1000:  1k 8.1 / 8.6,  5k 11.3 / 9.1,  20k 15.9 / 9.9;
+//                 with STDP 5k 23.5 / 11.0,  100k 52 / 25
+// and 110k neurons of mixed types with out-degrees of mean 50 up to 1000, a
+// tenth of them firing each step, 21.9 / 20.2: hence a bound on the largest
+// out-degree and one on the largest plastic in-degree.
+constexpr uint32_t LOCAL_MAX_OUT = 400;
+constexpr uint32_t LOCAL_MAX_IN = 320, LOCAL_MAX_IN_LARGE = 224, LOCAL_LARGE = 32768;
+// One cluster of 16 CTAs up to this many neurons: 1000 x 100 takes 3.24 us a
+// step against 3.60 with the grid barrier, 2000 x 100 3.38 against 3.67,
+// 5000 x 100 3.81 against 3.79 (with STDP 5.10 against 4.73).
+constexpr uint32_t LOCAL_CLUSTER_NEURONS = 2048, LOCAL_CLUSTER = 16;
+
+void Simulation::planLocal()
+{
+	for(const HostType& t : m_types) if(t.desc.kind == KIND_KURAMOTO) return;
+	if(!m_dev.dEnd16 || m_maxOutDeg > LOCAL_MAX_OUT) return;
+	if(m_dev.stdp && m_maxPlasticInDeg > (m_N <= LOCAL_LARGE ? LOCAL_MAX_IN : LOCAL_MAX_IN_LARGE)) return;
+	// rows of delay-group ends an odd number of words apart (bank conflicts)
+	m_localStride = (m_dev.dStride + 1) / 2 * 2;
+	if(m_localStride % 4 == 0) m_localStride += 2;
+	// workers, a noise warp for every two worker warps where they fit, the barrier warp
+	auto threads = [](uint32_t T) {
+		const int w = (int) T / 32;
+		return T + (uint32_t) std::max(1, std::min((w + 1) / 2, 31 - w)) * 32 + 32;
+	};
+	auto smem = [&](int sync, uint32_t T) {
+		return (size_t) T * (LOCAL_WORDS * 4 + m_localStride * 2 + (sync == 2 ? 0 : LOCAL_ACC * 4)) + (size_t) T / 32 * 2 * LOCAL_GROUPS * 4;
+	};
+	auto fits = [&](int sync, uint32_t T, uint32_t grid) -> bool {
+		for(bool serve : { false, true }) {
+			const void* k = local_kernel_for(sync, serve);
+			if(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) LOCAL_SMEM_MAX) != cudaSuccess) return false;
+			if(sync == 1) {
+				if(cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) return false;
+				cudaLaunchAttribute attr;
+				cudaLaunchConfig_t cfg = clusterConfig(grid, threads(T), smem(sync, T), attr);
+				int clusters = 0;
+				if(cudaOccupancyMaxActiveClusters(&clusters, k, &cfg) != cudaSuccess || clusters < 1) return false;
+			} else {
+				int perSm = 0;
+				if(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, k, (int) threads(T), smem(sync, T)) != cudaSuccess) return false;
+				if((uint64_t) perSm * m_sms < grid) return false;
+			}
+		}
+		return true;
+	};
+	auto plan = [&](int sync, uint32_t ctas) -> bool {
+		const uint32_t words = (m_dev.W + ctas - 1) / ctas, T = words * 32, grid = (m_dev.W + words - 1) / words;
+		if(threads(T) > LOCAL_THREADS || smem(sync, T) > LOCAL_SMEM_MAX) return false;
+		if(!fits(sync, T, grid)) {
+			cudaGetLastError();
+			return false;
+		}
+		m_localSync = sync;
+		m_localWorkers = T;
+		m_localT = threads(T);
+		m_localGrid = grid;
+		m_localSmem = smem(sync, T);
+		return true;
+	};
+	const bool cluster = m_N <= LOCAL_CLUSTER_NEURONS && maxInDegree() <= 65536 && plan(1, LOCAL_CLUSTER);
+	if(!cluster && !plan(2, (uint32_t) m_sms)) return;
+	if(m_localSync == 2) m_dev.slot2 = dalloc<ulonglong2>(2 * (size_t) m_N);
+	if(m_dev.stdp) m_dev.hist3 = dalloc<uint64_t>(3 * (size_t) m_N);
+	m_localOn = true;
+}
+
+// the largest in-degree over all synapses
+uint32_t Simulation::maxInDegree()
+{
+	auto* count = dalloc<uint32_t>((size_t) m_N + 1);
+	in_degree_kernel<<<592, 256, 0, m_stream>>>(m_dev.synTgt, m_nsyn, count);
+	max_kernel<<<1, 256, 0, m_stream>>>(count, m_N, count + m_N);
+	NB_CUDA(cudaGetLastError());
+	uint32_t most = 0;
+	NB_CUDA(cudaMemcpyAsync(&most, count + m_N, 4, cudaMemcpyDeviceToHost, m_stream));
+	NB_CUDA(cudaStreamSynchronize(m_stream));
+	return most;
+}
+
+cudaLaunchConfig_t Simulation::clusterConfig(unsigned grid, unsigned threads, size_t smem, cudaLaunchAttribute& attr) const
+{
+	cudaLaunchConfig_t cfg = {};
+	cfg.gridDim = dim3(grid);
+	cfg.blockDim = dim3(threads);
+	cfg.dynamicSmemBytes = smem;
+	cfg.stream = m_stream;
+	attr.id = cudaLaunchAttributeClusterDimension;
+	attr.val.clusterDim.x = grid;
+	attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+	cfg.attrs = &attr;
+	cfg.numAttrs = 1;
+	return cfg;
+}
+
+void Simulation::launchLocalKernel(bool serve, void** args)
+{
+	const void* k = local_kernel_for(m_localSync, serve);
+	if(m_localSync == 1) {
+		cudaLaunchAttribute attr;
+		const cudaLaunchConfig_t cfg = clusterConfig(m_localGrid, m_localT, m_localSmem, attr);
+		NB_CUDA(cudaLaunchKernelExC(&cfg, k, args));
+	} else {
+		NB_CUDA(cudaLaunchCooperativeKernel(k, dim3(m_localGrid), dim3(m_localT), args, m_localSmem, m_stream));
+	}
+	m_listsStale = true;
+}
+
+LocalLoop Simulation::localArgs(unsigned steps) const
+{
+	LocalLoop a = {};
+	a.steps = steps;
+	a.cycle0 = m_cycle;
+	a.gb = m_barrier;
+	a.workers = m_localWorkers;
+	a.rankMul = (uint32_t) ((0xffffffffull + m_localGrid) / m_localGrid);
+	a.rowStride = m_localStride;
+	return a;
+}
+
+// n consecutive steps in one launch of the single-barrier loop
+void Simulation::launchLocal(unsigned n)
+{
+	flushStdp();  // of a step of another loop
+	const uint64_t arrivals = m_localSync == 2 ? (uint64_t) m_localGrid * n : 0;
+	if(m_barrierStale || m_barrierBase + arrivals >= (1ull << 31)) {
+		NB_CUDA(cudaMemsetAsync(&m_barrier->count, 0, 4, m_stream));
+		m_barrierBase = 0;
+		m_barrierStale = false;
+	}
+	DevSim dev = m_dev;
+	LocalLoop a = localArgs(n);
+	a.base = (uint32_t) m_barrierBase;
+	void* args[] = { &dev, &a };
+	timedBegin(K_RUN);
+	launchLocalKernel(false, args);
+	timedEnd();
+	m_barrierBase += arrivals;
+	m_cycle += n;
+	m_timerSteps += n;
+	m_barrierUsed = true;
+}
+
+// After launches of the single-barrier loop: what the other loops' next step
+// expects from the last one's update.  Neither throws nor allocates (an
+// error surfaces at the next synchronisation).
+void Simulation::ensureLists() noexcept
+{
+	if(!m_listsStale) return;
+	m_listsStale = false;
+	stopServe();
+	cudaMemsetAsync(m_dev.dlvWork.count, 0, 16, m_stream);
+	cudaMemsetAsync(m_dev.stdpWork.count, 0, 16, m_stream);
+	publish_kernel<<<std::min(592u, (m_N + 255) / 256), 256, 0, m_stream>>>(m_dev, (uint32_t) ((m_cycle + 1) & 1));
+}
+
 void Simulation::setLaunch(uint32_t P, uint32_t T)
 {
 	stopServe();
 	if(persistentActive()) {
+		m_localOn = false;  // the caller shapes the persistent loop
 		// any multiple of 32 neurons per partition; 64 to RUN_THREADS threads
 		m_runP = std::max<uint32_t>(32, (std::min<uint32_t>(P, 1u << 30) + 31) & ~31u);
 		T = std::max<uint32_t>(64, std::min<uint32_t>(RUN_THREADS, (T + 31) & ~31u));
@@ -2219,6 +3109,7 @@ void Simulation::setLaunch(uint32_t P, uint32_t T)
 void Simulation::launchStep(bool /*fullRecord*/)
 {
 	stopServe();
+	ensureLists();
 	const uint32_t cur = (uint32_t) (m_cycle & 1);
 	const uint32_t ring = (uint32_t) (m_cycle % m_dev.R);
 	const unsigned grid = (m_N + m_P - 1) / m_P;
@@ -2266,6 +3157,7 @@ void Simulation::launchRun(unsigned n, bool finalStdp, const uint32_t* stim, uin
 	// it could wrap
 	const uint64_t arrivals = (uint64_t) grid * (2ull * n + (finalStdp ? 1 : 0));
 	stopServe();
+	ensureLists();
 	if(m_barrierStale || m_barrierBase + arrivals >= (1ull << 31)) {
 		NB_CUDA(cudaMemsetAsync(&m_barrier->count, 0, 4, m_stream));
 		m_barrierBase = 0;
@@ -2308,10 +3200,15 @@ void Simulation::checkBarrier()
 void Simulation::launchSteps(unsigned n)
 {
 	stopServe();
+	if(localActive()) {
+		launchLocal(n);
+		return;
+	}
 	if(usePersistent && m_runGrid && n > 1) {
 		launchRun(n);
 		return;
 	}
+	ensureLists();
 	if(!useGraphs || profiling || n < GRAPH_STEPS) {
 		for(unsigned i = 0; i < n; ++i) launchStep(false);
 		return;
@@ -2393,6 +3290,9 @@ void Simulation::launchServe()
 		NB_CUDA(cudaHostGetDevicePointer(&m_dFiredIdsMapped, m_hFiredIds, 0));
 	}
 	// the barrier counter and the request word (count and cmd, adjacent)
+	const bool local = localActive();
+	if(local) flushStdp();  // of a step of another loop
+	else ensureLists();
 	NB_CUDA(cudaMemsetAsync(&m_barrier->count, 0, 8, m_stream));
 	m_barrierBase = 0;
 	DevSim dev = m_dev;
@@ -2404,10 +3304,16 @@ void Simulation::launchServe()
 	const uint32_t* stim = m_dStimMapped;
 	uint32_t* hf = m_dFiredIdsMapped;
 	unsigned long long idleNs = (unsigned long long) residentIdleUs * 1000ull;
-	const unsigned grid = (unsigned) std::min<uint64_t>(m_runGrid, std::max<uint64_t>(1, (m_N + P - 1) / P));
-	void* args[] = { &dev, &P, &c0, &gb, &ctl, &seq0, &stim, &hf, &idleNs };
-	NB_CUDA(cudaLaunchCooperativeKernel(serve_kernel_for(m_runT), dim3(grid), dim3(m_runT), args, m_dev.recentBytes,
-			m_stream));
+	if(local) {
+		LocalLoop a = localArgs(0);
+		void* args[] = { &dev, &a, &ctl, &seq0, &stim, &hf, &idleNs };
+		launchLocalKernel(true, args);
+	} else {
+		const unsigned grid = (unsigned) std::min<uint64_t>(m_runGrid, std::max<uint64_t>(1, (m_N + P - 1) / P));
+		void* args[] = { &dev, &P, &c0, &gb, &ctl, &seq0, &stim, &hf, &idleNs };
+		NB_CUDA(cudaLaunchCooperativeKernel(serve_kernel_for(m_runT), dim3(grid), dim3(m_runT), args, m_dev.recentBytes,
+				m_stream));
+	}
 	NB_CUDA(cudaEventRecord(m_serveEnd, m_stream));
 	m_serving = true;
 	m_barrierUsed = true;
@@ -2475,7 +3381,7 @@ void Simulation::stepResident(uint32_t nf, uint32_t ni)
 	m_serveSeq = serve_next(m_serveSeq);
 	m_cycle++;
 	m_timerSteps++;
-	m_stdpPending = true;
+	m_stdpPending = !localActive();  // the single-barrier loop accumulates before it ends
 }
 
 // One step with host buffers: the stimulus is staged in mapped host memory
@@ -2530,6 +3436,7 @@ const std::vector<unsigned>& Simulation::step(const unsigned* fstim, size_t nf,
 	// slower here: its launch and grid barriers cost more than a second
 	// kernel)
 	stopServe();
+	ensureLists();
 	const uint32_t c = (uint32_t) (m_cycle & 1);
 	const uint32_t ring = (uint32_t) (m_cycle % m_dev.R);
 	launch_chained(deliver_kernel, m_deliverGrid, STEP_THREADS, m_dev.recentBytes, m_stream, m_dev, c ^ 1u,
@@ -2720,6 +3627,7 @@ void Simulation::collect(uint64_t first, unsigned chunk, unsigned begin, bool id
 float Simulation::autotune(unsigned trialSteps)
 {
 	NB_CUDA(cudaSetDevice(m_device));
+	ensureLists();
 	sync();
 	trialSteps = std::max(1u, trialSteps);
 	// the state that trial steps modify
@@ -2769,9 +3677,11 @@ float Simulation::autotune(unsigned trialSteps)
 		m_cycle = cycle;
 		m_timerSteps = timerSteps;
 		m_stdpPending = stdpPending;
+		m_listsStale = false;
 	};
 
 	std::vector<std::pair<uint32_t, uint32_t>> cands;
+	const bool local0 = m_localOn;
 	const bool pers = persistentActive();
 	if(pers) {
 		// persistent loop: 256 to RUN_THREADS threads per CTA, 1 to 4 partitions per CTA
@@ -2795,17 +3705,25 @@ float Simulation::autotune(unsigned trialSteps)
 			}
 		}
 	}
-	const uint32_t P0 = partition(), T0 = threads();
+	// the single-barrier loop (its own shape) against them
+	if(pers && m_localGrid) cands.emplace_back(0u, 0u);
+	const uint32_t P0 = pers ? m_runP : m_P, T0 = pers ? m_runT : m_T;
 	float best = -1;
 	uint32_t bestP = P0, bestT = T0;
+	bool bestLocal = local0;
 	try {
 		for(auto& c : cands) {
-			setLaunch(c.first, c.second);
+			const bool local = c.first == 0;
+			if(local) m_localOn = true;
+			else setLaunch(c.first, c.second);
 			// untimed warm-up of this shape
-			if(pers) launchRun(1);
+			if(local) launchLocal(1);
+			else if(pers) launchRun(1);
 			else launchStep(false);
 			NB_CUDA(cudaEventRecord(m_ev0, m_stream));
-			if(pers) {
+			if(local) {
+				launchLocal(trialSteps);
+			} else if(pers) {
 				launchRun(trialSteps);
 			} else {
 				for(unsigned i = 0; i < trialSteps; ++i) launchStep(false);
@@ -2818,8 +3736,11 @@ float Simulation::autotune(unsigned trialSteps)
 			NB_CUDA(cudaEventElapsedTime(&ms, m_ev0, m_ev1));
 			if(best < 0 || ms < best) {
 				best = ms;
-				bestP = partition();
-				bestT = threads();
+				bestLocal = local;
+				if(!local) {
+					bestP = partition();
+					bestT = threads();
+				}
 			}
 			restore();
 		}
@@ -2828,6 +3749,7 @@ float Simulation::autotune(unsigned trialSteps)
 		sync();
 		for(void* b : backup) if(b) cudaFree(b);
 		setLaunch(P0, T0);
+		m_localOn = local0;
 		profiling = prof;
 		throw;
 	}
@@ -2835,6 +3757,7 @@ float Simulation::autotune(unsigned trialSteps)
 	for(void* b : backup) if(b) cudaFree(b);
 	profiling = prof;
 	setLaunch(bestP, bestT);
+	m_localOn = pers ? bestLocal : local0;
 	return best * 1e3f / trialSteps;
 }
 

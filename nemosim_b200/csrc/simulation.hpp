@@ -117,6 +117,8 @@ struct DevSim {
 	uint32_t recentBytes;     // bytes of shared memory for the copy of one recent bit-vector (0 = none)
 	uint32_t* fstim;          // [W] pending firing stimulus
 	float* curExt;            // [N] pending current stimulus
+	ulonglong2* slot2;        // [2][N] the single-barrier loop's accumulators, by step parity (null: in shared memory)
+	uint64_t* hist3;          // [3][N] its histories for STDP, by cycle % 3
 	ulonglong2* slot;         // [N] int64 E and I fixed-point sums (two's complement) of this step's arrivals
 	const unsigned long long* outPtr; // [N+1] outgoing synapses per source, sorted by delay
 	uint32_t* synTgt;         // [S] target | (delay - 1) << 26
@@ -172,6 +174,17 @@ struct DevSim {
 // pre-phase, the release of the barrier after it, the end of the CTA's
 // update, and the release of the step's final barrier
 constexpr uint32_t TRACE_MARKS = 5;
+
+// arguments of the single-barrier step loop
+struct LocalLoop {
+	uint32_t steps;
+	unsigned long long cycle0;
+	GridBarrier* gb;
+	uint32_t base;       // SYNC 2: the barrier counter's value when the launch starts
+	uint32_t workers;    // neurons per CTA
+	uint32_t rankMul;    // ceil(2^32 / CTAs)
+	uint32_t rowStride;  // elements of a row of delay-group ends in shared memory
+};
 
 class Simulation {
 public:
@@ -232,10 +245,12 @@ public:
 	// launch shape of the active step loop (persistent or two-launch):
 	// partition size (neurons per partition; a CTA owns one or more) and
 	// threads per CTA; results do not depend on them
-	uint32_t partition() const { return persistentActive() ? m_runP : m_P; }
-	uint32_t threads() const { return persistentActive() ? m_runT : m_T; }
+	uint32_t partition() const { return localActive() ? m_localWorkers : persistentActive() ? m_runP : m_P; }
+	uint32_t threads() const { return localActive() ? m_localT : persistentActive() ? m_runT : m_T; }
 	void setLaunch(uint32_t P, uint32_t T);
 	bool persistentActive() const { return usePersistent && m_runGrid != 0; }
+	// the persistent loop's steps run through its single-barrier form
+	bool localActive() const { return persistentActive() && m_localOn; }
 	// step() keeps the persistent loop resident on the GPU between calls
 	// (serve_kernel) and ends it after this many microseconds without a
 	// call (at most RESIDENT_IDLE_MAX_US); 0: two kernel launches per step
@@ -333,6 +348,20 @@ private:
 	uint32_t m_runP = 0;     // neurons per partition of run_kernel
 	uint32_t m_runT = 384;
 	unsigned runGridFor(uint32_t T) const;
+	// the single-barrier loop: whether it is in use, its CTAs' way to wait
+	// (LoopBarrier), neurons and threads per CTA, CTAs, shared memory, row stride
+	bool m_localOn = false;
+	int m_localSync = 2;
+	uint32_t m_localWorkers = 0, m_localT = 0, m_localGrid = 0, m_localStride = 0;
+	size_t m_localSmem = 0;
+	bool m_listsStale = false;  // its launches left the other loops' work lists behind
+	void planLocal();
+	uint32_t maxInDegree();
+	LocalLoop localArgs(unsigned steps) const;
+	cudaLaunchConfig_t clusterConfig(unsigned grid, unsigned threads, size_t smem, cudaLaunchAttribute& attr) const;
+	void launchLocalKernel(bool serve, void** args);
+	void launchLocal(unsigned n);
+	void ensureLists() noexcept;
 	void buildGraph();
 	static constexpr unsigned GRAPH_STEPS = 100;
 	cudaGraphExec_t m_graph = nullptr;
