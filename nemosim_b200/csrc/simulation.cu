@@ -1687,6 +1687,103 @@ local_serve_kernel(const DevSim S, const LocalLoop A, ServeCtl* ctl, uint32_t se
 	bar.finish();
 }
 
+// The same step for networks beyond the loop's resident threads (a large
+// batch): one launch a step, its end the barrier, one neuron per thread with
+// its state in global memory.  After its update a warp delivers its own
+// neurons' groups for the next step and accumulates STDP for its targets, so
+// a step needs neither work lists nor their reservations, and deliveries
+// overlap the updates of other warps: 24 networks of 400k neurons and 80M
+// synapses take 18.8 us a step, against 29.8 with deliver_kernel and
+// update_kernel at two partitions per SM and 23.0 at one of 128 neurons per
+// CTA.  The noise comes from the libm tables (evaluated: 20.9).
+// deliver: not in the last step before applyStdp may run.
+__global__ void __launch_bounds__(FUSED_THREADS, 8)
+fused_step_kernel(const DevSim S, uint32_t cur, uint32_t ring, uint32_t offset, int fromDev, int deliver)
+{
+	chain_wait_then_release();
+	uint32_t cycleLo;
+	if(fromDev) step_indices(S, offset, cur, ring, cycleLo);
+	__shared__ uint32_t sLists[FUSED_THREADS / 32 * 2 * LOCAL_GROUPS];
+	__shared__ LocalCounters sC;
+	if(threadIdx.x == 0) sC = LocalCounters{ 0, 0, 0 };
+	__syncthreads();
+	const uint32_t n = blockIdx.x * FUSED_THREADS + threadIdx.x, lane = threadIdx.x & 31;
+	LocalNeuron L;
+	L.list = sLists + (threadIdx.x >> 5) * 2 * LOCAL_GROUPS;
+	L.h = L.dm = 0;
+	L.ob = L.outdeg = L.rb = L.indeg = 0;
+	L.ends = nullptr;
+	bool fired = false, target = false;
+	if(n < S.N) {
+		const TypeRange& T = local_type(S, n);
+		const uint32_t nl = n - T.base;
+		ulonglong2* slot = S.slot2 + (size_t) cur * S.N + n;
+		const ulonglong2 acc = *slot;
+		const uint64_t hp = S.hist[(size_t) (cur ^ 1u) * S.N + n];
+		L.dm = S.delayMask[n];
+		const unsigned long long o0 = S.outPtr[n], o1 = S.outPtr[n + 1];
+		if(S.stdp) {
+			L.rb = (uint32_t) S.rcmPtr[n];
+			L.indeg = (uint32_t) (S.rcmPtr[n + 1] - S.rcmPtr[n]);
+		}
+		NeuronRegs R;
+		load_neuron(S, T, nl, n, R, false);
+		L.ob = (uint32_t) o0;
+		L.outdeg = (uint32_t) (o1 - o0);
+		L.ends = S.dEnd16 + (size_t) n * S.dStride;
+		if(acc.x | acc.y) *slot = make_ulonglong2(0, 0);
+		fired = update_neuron(S, T, R, wfx_to_float((long long) acc.x), wfx_to_float((long long) acc.y), 0.0f, false);
+		store_neuron(S, T, nl, n, R);
+		L.h = (hp << 1) | (uint64_t) fired;
+		S.hist[(size_t) cur * S.N + n] = L.h;
+		target = S.stdp && (L.h & S.sp.postFireMask) && L.indeg > 0;
+	}
+	const uint32_t fb = __ballot_sync(0xffffffffu, fired);
+	if(lane == 0 && n < S.N) S.firedRing[(size_t) ring * S.W + (n >> 5)] = fb;
+	if(deliver) local_deliver<2>(S, L, cur ^ 1u, 0, L.h & L.dm);
+	if(fb) {
+		const uint32_t ev = __reduce_add_sync(0xffffffffu, fired ? L.outdeg : 0u);
+		if(lane == 0) {
+			atomicAdd(&sC.fired, (uint32_t) __popc(fb));
+			atomicAdd(&sC.events, ev);
+		}
+	}
+	const uint32_t tb = __ballot_sync(0xffffffffu, target);
+	if(tb) {
+		const uint32_t se = __reduce_add_sync(0xffffffffu, target ? L.indeg : 0u);
+		if(lane == 0) {
+			atomicOr(&S.touchedBits[n >> 5], tb);
+			atomicAdd(&sC.stdp, se);
+		}
+		local_stdp(S, L, target, S.hist + (size_t) (cur ^ 1u) * S.N);
+	}
+	__syncthreads();
+	if(threadIdx.x == 0) flush_counters(S, ring, sC);
+}
+
+// the deliveries to the first of a sequence of those steps
+__global__ void __launch_bounds__(FUSED_THREADS, 8)
+fused_deliver_kernel(const DevSim S, uint32_t cur, int fromDev)
+{
+	chain_wait_then_release();
+	uint32_t ring, cycleLo;
+	if(fromDev) step_indices(S, 0, cur, ring, cycleLo);
+	__shared__ uint32_t sLists[FUSED_THREADS / 32 * 2 * LOCAL_GROUPS];
+	const uint32_t n = blockIdx.x * FUSED_THREADS + threadIdx.x;
+	LocalNeuron L;
+	L.list = sLists + (threadIdx.x >> 5) * 2 * LOCAL_GROUPS;
+	L.h = L.dm = 0;
+	L.ob = 0;
+	L.ends = nullptr;
+	if(n < S.N) {
+		L.h = S.hist[(size_t) (cur ^ 1u) * S.N + n];
+		L.dm = S.delayMask[n];
+		L.ob = (uint32_t) S.outPtr[n];
+		L.ends = S.dEnd16 + (size_t) n * S.dStride;
+	}
+	local_deliver<2>(S, L, cur, 0, L.h & L.dm);
+}
+
 __global__ void in_degree_kernel(const uint32_t* synTgt, size_t n, uint32_t* count)
 {
 	for(size_t i = (size_t) blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t) gridDim.x * blockDim.x) {
@@ -2816,9 +2913,15 @@ void Simulation::init(const std::vector<const Network*>& nets, const Configurati
 		// the persistent loop's CTAs are those that fit at once; when each
 		// thread would update more than two neurons in turn, the update is
 		// faster as one launch over the whole network (a large batch)
-		if((uint64_t) N > 2ull * m_runGrid * m_runT) usePersistent = false;
+		if((uint64_t) N > 2ull * m_runGrid * m_runT) {
+			usePersistent = false;
+			// one neuron per thread in many small CTAs, against two
+			// partitions per SM: 23.0 / 29.8 us a step at 400k neurons
+			setLaunch(128, 128);
+		}
 		if(m_runGrid) planLocal();
 	}
+	planFused();
 	NB_CUDA(cudaStreamSynchronize(m_stream));
 	resetTimer();
 }
@@ -2934,6 +3037,8 @@ unsigned Simulation::runGridFor(uint32_t T) const
 // out-degree and one on the largest plastic in-degree.
 constexpr uint32_t LOCAL_MAX_OUT = 400;
 constexpr uint32_t LOCAL_MAX_IN = 320, LOCAL_MAX_IN_LARGE = 224, LOCAL_LARGE = 32768;
+// the fused step (planFused)
+constexpr uint32_t FUSED_MAX_OUT_LARGE = 640, FUSED_LARGE = 900000;
 // One cluster of 16 CTAs up to this many neurons: 1000 x 100 takes 3.24 us a
 // step against 3.60 with the grid barrier, 2000 x 100 3.38 against 3.67,
 // 5000 x 100 3.81 against 3.79 (with STDP 5.10 against 4.73).
@@ -3098,6 +3203,7 @@ void Simulation::setLaunch(uint32_t P, uint32_t T)
 		}
 		return;
 	}
+	m_fusedOn = false;  // the caller shapes the two-launch step
 	P = std::max<uint32_t>(32, std::min<uint32_t>(MAX_PARTITION, (P + 31) & ~31u));
 	T = std::max<uint32_t>(32, std::min<uint32_t>(1024, (T + 31) & ~31u));
 	// the per-CTA work offsets are 32-bit
@@ -3208,40 +3314,97 @@ void Simulation::launchSteps(unsigned n)
 		launchRun(n);
 		return;
 	}
-	ensureLists();
+	const bool fused = !persistentActive() && m_fusedOn;
+	if(fused) {
+		flushStdp();  // of a step of another loop
+		m_listsStale = true;
+	} else {
+		ensureLists();
+	}
+	auto single = [&](unsigned count) {
+		if(fused) {
+			launchFused(count);
+		} else {
+			for(unsigned i = 0; i < count; ++i) launchStep(false);
+		}
+	};
 	if(!useGraphs || profiling || n < GRAPH_STEPS) {
-		for(unsigned i = 0; i < n; ++i) launchStep(false);
+		single(n);
 		return;
 	}
-	if(!m_graph || m_graphP != m_P || m_graphT != m_T) buildGraph();
+	buildGraph();
 	*m_hCycle = m_cycle;
 	NB_CUDA(cudaMemcpyAsync(m_dev.cycleDev, m_hCycle, 8, cudaMemcpyHostToDevice, m_stream));
 	while(n >= GRAPH_STEPS) {
 		NB_CUDA(cudaGraphLaunch(m_graph, m_stream));
 		m_cycle += GRAPH_STEPS;
 		m_timerSteps += GRAPH_STEPS;
-		m_stdpPending = true;
+		m_stdpPending = !fused;
 		n -= GRAPH_STEPS;
 	}
 	// the pinned cycle value must not change before the copy above ran
 	NB_CUDA(cudaStreamSynchronize(m_stream));
-	for(unsigned i = 0; i < n; ++i) launchStep(false);
+	if(n) single(n);
 }
 
+// n consecutive steps of fused_step_kernel, one launch each
+void Simulation::launchFused(unsigned n)
+{
+	const unsigned grid = (m_N + FUSED_THREADS - 1) / FUSED_THREADS;
+	timedBegin(K_STDP);
+	launch_chained(fused_deliver_kernel, grid, FUSED_THREADS, 0, m_stream, m_dev, (uint32_t) (m_cycle & 1), 0);
+	timedEnd();
+	for(unsigned i = 0; i < n; ++i) {
+		timedBegin(K_STEP);
+		launch_chained(fused_step_kernel, grid, FUSED_THREADS, 0, m_stream, m_dev, (uint32_t) (m_cycle & 1),
+				(uint32_t) (m_cycle % m_dev.R), 0u, 0, (int) (i + 1 < n));
+		timedEnd();
+		m_cycle++;
+		m_timerSteps++;
+	}
+}
+
+// Whether the two-launch step runs as one kernel: the single-barrier loop's
+// types, and degrees small enough for one warp beside the other work of a
+// step.  Microseconds a step, fused / two launches (batches of equal example
+// networks, delays to 20 ms):
+//   300k neurons, fan-out 100 12.9 / 17.9, 300 16.8 / 19.7, 600 24.8 / 23.8, 1000 37.4 / 30.4;
+//   with STDP 100 17.7 / 22.2, 300 27.4 / 25.4;
+//   960k neurons, 600 60.5 / 68.4;  with STDP 100 51.3 / 55.1, 600 101 / 85
+void Simulation::planFused()
+{
+	for(const HostType& t : m_types) if(t.desc.kind == KIND_KURAMOTO) return;
+	if(!m_dev.dEnd16 || m_maxOutDeg > (m_N >= FUSED_LARGE ? FUSED_MAX_OUT_LARGE : LOCAL_MAX_OUT)) return;
+	if(m_maxPlasticInDeg > LOCAL_MAX_IN_LARGE) return;
+	if(!m_dev.slot2) m_dev.slot2 = dalloc<ulonglong2>(2 * (size_t) m_N);
+	m_fusedOn = m_fusedFits = true;
+}
+
+// the graph of GRAPH_STEPS two-launch (or fused) steps for the current shape
 void Simulation::buildGraph()
 {
+	const uint32_t P = m_fusedOn ? 0u : m_P, T = m_fusedOn ? 0u : m_T;
+	if(m_graph && m_graphP == P && m_graphT == T) return;
 	if(m_graph) {
 		cudaGraphExecDestroy(m_graph);
 		m_graph = nullptr;
 	}
 	sync();
-	const unsigned grid = (m_N + m_P - 1) / m_P;
 	cudaGraph_t g;
 	NB_CUDA(cudaStreamBeginCapture(m_stream, cudaStreamCaptureModeThreadLocal));
-	for(unsigned k = 0; k < GRAPH_STEPS; ++k) {
-		launch_chained(deliver_kernel, m_deliverGrid, STEP_THREADS, m_dev.recentBytes, m_stream, m_dev, 0u,
-				(uint32_t) (PHASE_DELIVER | PHASE_STDP | PHASE_RESET), k, 1, nullptr, 0u, 0u);
-		launch_chained(update_kernel_for(m_T), grid, m_T, 0, m_stream, m_dev, m_P, 0u, 0u, 0u, k, 1, nullptr);
+	if(m_fusedOn) {
+		const unsigned grid = (m_N + FUSED_THREADS - 1) / FUSED_THREADS;
+		launch_chained(fused_deliver_kernel, grid, FUSED_THREADS, 0, m_stream, m_dev, 0u, 1);
+		for(unsigned k = 0; k < GRAPH_STEPS; ++k) {
+			launch_chained(fused_step_kernel, grid, FUSED_THREADS, 0, m_stream, m_dev, 0u, 0u, k, 1, (int) (k + 1 < GRAPH_STEPS));
+		}
+	} else {
+		const unsigned grid = (m_N + m_P - 1) / m_P;
+		for(unsigned k = 0; k < GRAPH_STEPS; ++k) {
+			launch_chained(deliver_kernel, m_deliverGrid, STEP_THREADS, m_dev.recentBytes, m_stream, m_dev, 0u,
+					(uint32_t) (PHASE_DELIVER | PHASE_STDP | PHASE_RESET), k, 1, nullptr, 0u, 0u);
+			launch_chained(update_kernel_for(m_T), grid, m_T, 0, m_stream, m_dev, m_P, 0u, 0u, 0u, k, 1, nullptr);
+		}
 	}
 	advance_cycle_kernel<<<1, 1, 0, m_stream>>>(m_dev.cycleDev, GRAPH_STEPS);
 	NB_CUDA(cudaStreamEndCapture(m_stream, &g));
@@ -3251,8 +3414,8 @@ void Simulation::buildGraph()
 		m_graph = nullptr;
 		NB_THROW(NEMO_CUDA_ERROR, "CUDA graph instantiation failed: %s", cudaGetErrorString(err));
 	}
-	m_graphP = m_P;
-	m_graphT = m_T;
+	m_graphP = P;
+	m_graphT = T;
 }
 
 // ---------------------------------------------------------------------------
@@ -3517,10 +3680,7 @@ void Simulation::run(unsigned steps, unsigned stdpPeriod, float reward, unsigned
 	// the two-launch loop's CUDA graph is instantiated (once per launch
 	// shape) before the run's timing events, which time the simulation only
 	const unsigned longest = stdpPeriod ? std::min(stdpPeriod, steps) : steps;
-	if(!persistentActive() && useGraphs && !profiling && longest >= GRAPH_STEPS
-			&& (!m_graph || m_graphP != m_P || m_graphT != m_T)) {
-		buildGraph();
-	}
+	if(!persistentActive() && useGraphs && !profiling && longest >= GRAPH_STEPS) buildGraph();
 	size_t total = 0;
 	float runMs = 0;
 	for(int k = 0; k < K_KINDS; ++k) { kernelMs[k] = 0; kernelLaunches[k] = 0; }
@@ -3705,24 +3865,34 @@ float Simulation::autotune(unsigned trialSteps)
 			}
 		}
 	}
-	// the single-barrier loop (its own shape) against them
-	if(pers && m_localGrid) cands.emplace_back(0u, 0u);
+	// the single-barrier loop or the fused step (their own shapes) against them
+	const bool fused0 = m_fusedOn;
+	if(pers ? m_localGrid != 0 : m_fusedFits) cands.emplace_back(0u, 0u);
 	const uint32_t P0 = pers ? m_runP : m_P, T0 = pers ? m_runT : m_T;
 	float best = -1;
 	uint32_t bestP = P0, bestT = T0;
-	bool bestLocal = local0;
+	bool bestLocal = false;
 	try {
 		for(auto& c : cands) {
 			const bool local = c.first == 0;
-			if(local) m_localOn = true;
-			else setLaunch(c.first, c.second);
+			if(!local) setLaunch(c.first, c.second);
+			else if(pers) m_localOn = true;
+			else m_fusedOn = true;
+			auto own = [&](unsigned n) {
+				if(pers) {
+					launchLocal(n);
+				} else {
+					flushStdp();
+					launchFused(n);
+				}
+			};
 			// untimed warm-up of this shape
-			if(local) launchLocal(1);
+			if(local) own(1);
 			else if(pers) launchRun(1);
 			else launchStep(false);
 			NB_CUDA(cudaEventRecord(m_ev0, m_stream));
 			if(local) {
-				launchLocal(trialSteps);
+				own(trialSteps);
 			} else if(pers) {
 				launchRun(trialSteps);
 			} else {
@@ -3750,6 +3920,7 @@ float Simulation::autotune(unsigned trialSteps)
 		for(void* b : backup) if(b) cudaFree(b);
 		setLaunch(P0, T0);
 		m_localOn = local0;
+		m_fusedOn = fused0;
 		profiling = prof;
 		throw;
 	}
@@ -3758,6 +3929,7 @@ float Simulation::autotune(unsigned trialSteps)
 	profiling = prof;
 	setLaunch(bestP, bestT);
 	m_localOn = pers ? bestLocal : local0;
+	m_fusedOn = pers ? fused0 : bestLocal;
 	return best * 1e3f / trialSteps;
 }
 

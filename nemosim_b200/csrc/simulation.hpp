@@ -21,6 +21,8 @@ constexpr unsigned STEP_THREADS = 256;   // block size of the apply/stimulus ker
 constexpr unsigned MAX_PARTITION = 2048; // neurons per CTA of the step kernel
 constexpr unsigned RUN_THREADS = 768;    // largest block of the persistent step loop (registers for 768 x 1 or 384 x 2 per SM)
 
+constexpr unsigned FUSED_THREADS = 128;  // neurons per CTA of the fused step
+
 // Grid barrier of the persistent step loop (device memory; the counter is
 // zeroed before each launch, the error word when the host has read it).
 struct GridBarrier {
@@ -245,8 +247,8 @@ public:
 	// launch shape of the active step loop (persistent or two-launch):
 	// partition size (neurons per partition; a CTA owns one or more) and
 	// threads per CTA; results do not depend on them
-	uint32_t partition() const { return localActive() ? m_localWorkers : persistentActive() ? m_runP : m_P; }
-	uint32_t threads() const { return localActive() ? m_localT : persistentActive() ? m_runT : m_T; }
+	uint32_t partition() const { return localActive() ? m_localWorkers : persistentActive() ? m_runP : m_fusedOn ? FUSED_THREADS : m_P; }
+	uint32_t threads() const { return localActive() ? m_localT : persistentActive() ? m_runT : m_fusedOn ? FUSED_THREADS : m_T; }
 	void setLaunch(uint32_t P, uint32_t T);
 	bool persistentActive() const { return usePersistent && m_runGrid != 0; }
 	// the persistent loop's steps run through its single-barrier form
@@ -361,6 +363,10 @@ private:
 	cudaLaunchConfig_t clusterConfig(unsigned grid, unsigned threads, size_t smem, cudaLaunchAttribute& attr) const;
 	void launchLocalKernel(bool serve, void** args);
 	void launchLocal(unsigned n);
+	// the two-launch step as one kernel (fused_step_kernel): in use, possible
+	bool m_fusedOn = false, m_fusedFits = false;
+	void planFused();
+	void launchFused(unsigned n);
 	void ensureLists() noexcept;
 	void buildGraph();
 	static constexpr unsigned GRAPH_STEPS = 100;

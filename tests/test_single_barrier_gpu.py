@@ -152,3 +152,29 @@ def test_many_synapses_onto_one_neuron():
     co, io = so.run(40, max_ids=40 * 210)
     assert np.array_equal(cp, co) and np.array_equal(ip, io)
     assert np.array_equal(sp.type_state(1, 2, 10).view(np.uint32), so.type_state(1, 2, 10).view(np.uint32))
+
+
+@pytest.mark.parametrize("stdp", [True, False])
+@pytest.mark.parametrize("n", [1, 127, 129, 3000])
+def test_fused_step_matches_oracle(n, stdp):
+    """The same step as one kernel per step (two-launch mode): without and
+    with graphs of 100 steps, and followed by the other loops."""
+    fanout = min(n, 40)
+    (pn, parts), (on, _) = typed_network(nb, n, fanout, 25, 0.1, 6), typed_network(O, n, fanout, 25, 0.1, 6)
+    sp, so = nb.Simulation(pn, conf(nb, stdp)), O.Simulation(on, conf(O, stdp))
+    sp.set_persistent(False)
+    for k, steps in enumerate((1, 2, 99, 100, 231, 30)):
+        if k == 4:
+            sp.set_graphs(False)
+        if k == 5:
+            sp.set_persistent(True)
+        period = 110 if stdp else 0
+        cp, _, ip = sp.run(steps, period, 0.7, max_ids=steps * n + 1)
+        co, io = so.run(steps, period, 0.7, max_ids=steps * n + 1)
+        assert np.array_equal(cp, co) and np.array_equal(ip, io)
+        got, want = sp.step([int(parts[0][0])] if len(parts[0]) else None), so.step([int(parts[0][0])] if len(parts[0]) else None)
+        assert list(got) == list(want)
+        sp.set_persistent(k >= 4)
+    assert_same_state(sp, so, parts)
+    if stdp:
+        assert np.array_equal(sp.weights_fx(n * fanout), so.weights_fx(n * fanout))
