@@ -177,6 +177,9 @@ struct DevSim {
 // update, and the release of the step's final barrier
 constexpr uint32_t TRACE_MARKS = 5;
 
+// m_localSync of the balanced form (two barriers, work lists)
+constexpr int LOCAL_BALANCED = 3;
+
 // arguments of the single-barrier step loop
 struct LocalLoop {
 	uint32_t steps;
@@ -186,6 +189,7 @@ struct LocalLoop {
 	uint32_t workers;    // neurons per CTA
 	uint32_t rankMul;    // ceil(2^32 / CTAs)
 	uint32_t rowStride;  // elements of a row of delay-group ends in shared memory
+	uint32_t recentAt;   // balanced form: offset of the STDP filter in shared memory
 };
 
 class Simulation {

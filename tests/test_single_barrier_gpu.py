@@ -133,6 +133,32 @@ def test_degree_limit(fanout):
     assert np.array_equal(cp, co) and np.array_equal(ip, io)
 
 
+@pytest.mark.parametrize("n,fanout,dmax,rate,stdp", [
+    (3, 450, 5, 0.5, True), (33, 401, 44, 0.3, True), (700, 500, 20, 0.05, False), (4737, 410, 40, 0.02, True),
+    (300, 420, 63, 1.0, False), (300, 420, 44, 1.0, True)])
+def test_balanced_form_matches_oracle(n, fanout, dmax, rate, stdp):
+    """The two-barrier form of large degrees, with steps between runs."""
+    (pn, parts), (on, _) = typed_network(nb, n, fanout, dmax, rate, 8), typed_network(O, n, fanout, dmax, rate, 8)
+    sp, so = nb.Simulation(pn, conf(nb, stdp)), O.Simulation(on, conf(O, stdp))
+    ids = np.concatenate(parts)
+    for k, steps in enumerate((1, 2, 57, 40)):
+        cp, _, ip = sp.run(steps, 19 if stdp else 0, 0.7, max_ids=steps * n + 1)
+        co, io = so.run(steps, 19 if stdp else 0, 0.7, max_ids=steps * n + 1)
+        assert np.array_equal(cp, co) and np.array_equal(ip, io)
+        for j in range(5):
+            i = [(int(ids[j % n]), 15.0)]
+            assert list(sp.step([int(ids[0])], i)) == list(so.step([int(ids[0])], i))
+        if k == 1:
+            assert list(sp.step_no_alloc()[1]) == list(so.step())
+        if k == 2:
+            sp.set_persistent(False)
+            assert list(sp.run(9, max_ids=9 * n + 1)[2]) == list(so.run(9, max_ids=9 * n + 1)[1])
+            sp.set_persistent(True)
+    assert_same_state(sp, so, parts)
+    if stdp:
+        assert np.array_equal(sp.weights_fx(n * fanout), so.weights_fx(n * fanout))
+
+
 def test_many_synapses_onto_one_neuron():
     """A target whose in-degree exceeds the 65536 arrivals of the cluster's
     split sums, all of them in the same step, with weights of both signs and
