@@ -772,17 +772,14 @@ run_kernel(const DevSim S, uint32_t P, uint32_t steps, unsigned long long cycle0
 // call costs a step and a round trip through host memory instead of kernel
 // launches and a stream synchronisation.
 //
-// The host writes the step's stimulus (stim, mapped host memory), its sizes
-// and then the request's sequence number to ctl->go.  Thread 0 of CTA 0
-// polls ctl->go and broadcasts the request (its sequence number) through
-// gb->cmd, which the other CTAs poll.  After the step's final barrier CTA 0
-// writes the step's fired neurons as global ids to hostIds (mapped), their
-// number and the step's synaptic events to ctl, and then the sequence
-// number to ctl->done.  The loop ends when the host asks it to stop
-// (go = the next sequence number | SERVE_STOP) or after idleNs nanoseconds
-// without a request (the host then launches it again for the next call);
-// a wait that gives up ends it with the barrier's error word set.  Step k
-// runs cycle cycle0 + k, exactly as run_kernel's step.
+// The host writes the step's stimulus (stim, mapped host memory) and then the
+// request line.  Warp 0 of CTA 0 polls it and broadcasts the request (its
+// sequence number) through gb->cmd, which the other CTAs poll.  After the
+// step's final barrier CTA 0 answers (answer_request).  The loop ends when the
+// host asks it to stop (the next sequence number | SERVE_STOP) or after idleNs
+// nanoseconds without a request (the host then launches it again for the next
+// call); a wait that gives up ends it with the barrier's error word set.
+// Step k runs cycle cycle0 + k, exactly as run_kernel's step.
 constexpr uint32_t SERVE_POLL_LIMIT = 1u << 26;  // bounds the idle wait even without the timer
 
 
@@ -792,11 +789,6 @@ __device__ __forceinline__ unsigned long long ld_relaxed_sys_u64(const unsigned 
 	unsigned long long v;
 	asm volatile("ld.relaxed.sys.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
 	return v;
-}
-
-__device__ __forceinline__ void st_release_sys(uint32_t* p, uint32_t v)
-{
-	asm volatile("st.release.sys.u32 [%0], %1;" :: "l"(p), "r"(v) : "memory");
 }
 
 // n words from device memory (just written by other CTAs: read from L2)
@@ -819,20 +811,40 @@ __device__ __forceinline__ void st_release(uint32_t* p, uint32_t v)
 	asm volatile("st.release.gpu.global.u32 [%0], %1;" :: "l"(p), "r"(v) : "memory");
 }
 
-// The fired neurons of a step (words: its fired bit-vector) as global ids in
-// ascending local index (setFiring, src/nemo/cpu/Simulation.cpp:200-208),
-// by the threads of one CTA: each thread takes a run of words, a CTA-wide
-// scan of their counts places its ids, which are staged in shared memory
-// (or, beyond SERVE_IDS_SMEM of them, in S.firedIds) and then stored to host
-// memory in consecutive words per warp.  Returns the count.
-constexpr uint32_t SERVE_IDS_SMEM = 4096;
-
-__device__ uint32_t fired_ids_to_host(const DevSim& S, const uint32_t* words, uint32_t* host)
+// Answers request `want` with the fired neurons of its step (ring row `ring`) as
+// global ids in ascending local index (setFiring, src/nemo/cpu/
+// Simulation.cpp:200-208) and its synaptic events, by the threads of CTA 0.
+// Up to SERVE_TAGGED ids travel like an inline stimulus: every 8-byte word of
+// the answer carries the request's sequence number, and the host takes each
+// word as it arrives, so nothing waits until the writes have reached host
+// memory (a release at system scope took 1.4 to 1.9 us).  More ids go to
+// hostIds, published by such a release.
+__device__ void answer_request(const DevSim& S, ServeCtl* ctl, uint32_t ring, uint32_t* hostIds, uint32_t want)
 {
-	__shared__ uint32_t sIds[SERVE_IDS_SMEM];
+	const uint32_t* words = S.firedRing + (size_t) ring * S.W;
+	const unsigned long long tag = (unsigned long long) want << 32;
+	const uint32_t T = blockDim.x, t = threadIdx.x, lane = t & 31, warp = t >> 5;
+	auto global_id = [&](uint32_t l) { return S.l2gIdentity ? l : __ldg(S.l2g + l); };
+	// fewer events than the network's synapses, which are fewer than 2^32
+	unsigned long long events = 0;
+	if(t == 0) events = *(volatile unsigned long long*) &S.eventCount[ring];
+	if(S.W <= 32) {
+		if(warp == 0) {
+			uint32_t bits = lane < S.W ? __ldcg(words + lane) : 0u;
+			const uint32_t n = __popc(bits), incl = warp_inclusive_scan(n);
+			uint32_t pos = incl - n;
+			for(; bits; bits &= bits - 1) ctl->ids[pos++] = tag | global_id(lane * 32 + __ffs(bits) - 1);
+			const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
+			if(lane == 0) {
+				ctl->reply[0] = tag | total;
+				ctl->reply[1] = tag | (uint32_t) events;
+			}
+		}
+		return;
+	}
+	__shared__ uint32_t sIds[SERVE_TAGGED];
 	__shared__ uint32_t sWarp[32];
 	__shared__ uint32_t sTotal;
-	const uint32_t T = blockDim.x, t = threadIdx.x, lane = t & 31, warp = t >> 5;
 	const uint32_t per = (S.W + T - 1) / T;
 	const uint32_t w0 = min(S.W, t * per), w1 = min(S.W, w0 + per);
 	// up to WREG words per thread stay in registers for the second pass
@@ -857,43 +869,34 @@ __device__ uint32_t fired_ids_to_host(const DevSim& S, const uint32_t* words, ui
 	__syncthreads();
 	const uint32_t total = sTotal;
 	uint32_t pos = sWarp[warp] + incl - n;
-	if(total <= SERVE_IDS_SMEM) {
+	if(total <= SERVE_TAGGED) {
+		if(t == 0) {
+			ctl->reply[0] = tag | total;
+			ctl->reply[1] = tag | (uint32_t) events;
+		}
 #pragma unroll
 		for(uint32_t j = 0; j < WREG; ++j) {
-			uint32_t bits = wr[j];
-			while(bits) {
-				const uint32_t b = __ffs(bits) - 1;
-				bits &= bits - 1;
-				sIds[pos++] = (w0 + j) * 32 + b;
-			}
+			for(uint32_t bits = wr[j]; bits; bits &= bits - 1) sIds[pos++] = (w0 + j) * 32 + __ffs(bits) - 1;
 		}
 		for(uint32_t w = w0 + WREG; w < w1; ++w) {
-			uint32_t bits = __ldcg(words + w);
-			while(bits) {
-				const uint32_t b = __ffs(bits) - 1;
-				bits &= bits - 1;
-				sIds[pos++] = w * 32 + b;
-			}
+			for(uint32_t bits = __ldcg(words + w); bits; bits &= bits - 1) sIds[pos++] = w * 32 + __ffs(bits) - 1;
 		}
 		__syncthreads();
-		if(S.l2gIdentity) {
-			for(uint32_t i = t; i < total; i += T) host[i] = sIds[i];
-		} else {
-			for(uint32_t i = t; i < total; i += T) host[i] = __ldg(S.l2g + sIds[i]);
-		}
-		return total;
+		for(uint32_t i = t; i < total; i += T) ctl->ids[i] = tag | global_id(sIds[i]);
+		return;
 	}
 	for(uint32_t w = w0; w < w1; ++w) {
-		uint32_t bits = __ldcg(words + w);
-		while(bits) {
-			const uint32_t b = __ffs(bits) - 1;
-			bits &= bits - 1;
-			S.firedIds[pos++] = S.l2g[w * 32 + b];
-		}
+		for(uint32_t bits = __ldcg(words + w); bits; bits &= bits - 1) S.firedIds[pos++] = S.l2g[w * 32 + __ffs(bits) - 1];
 	}
 	__syncthreads();
-	copy_words_to_host(S.firedIds, host, total);
-	return total;
+	copy_words_to_host(S.firedIds, hostIds, total);
+	__syncthreads();
+	if(t == 0) {
+		ctl->reply[1] = tag | (uint32_t) events;
+		// a release at system scope: the host that sees the word sees every
+		// store the CTA made before the __syncthreads
+		asm volatile("st.release.sys.u64 [%0], %1;" :: "l"(&ctl->reply[0]), "l"(tag | total) : "memory");
+	}
 }
 
 // A CTA other than 0 waits for CTA 0's broadcast of request `want` (1) or
@@ -1012,15 +1015,7 @@ serve_kernel(const DevSim S, uint32_t P, unsigned long long cycle0, GridBarrier*
 		// CTA 0 answers: the step's fired ids and events (after the step's
 		// final barrier every CTA's words and counts are in place)
 		if(blockIdx.x == 0) {
-			const uint32_t n = fired_ids_to_host(S, S.firedRing + (size_t) ring * S.W, hostIds);
-			__syncthreads();
-			if(threadIdx.x == 0) {
-				ctl->fired = n;
-				ctl->events = *(volatile unsigned long long*) &S.eventCount[ring];
-				// a release at system scope: the host that sees done sees
-				// every store the CTA made before the __syncthreads
-				st_release_sys(&ctl->done, want);
-			}
+			answer_request(S, ctl, ring, hostIds, want);
 		}
 	}
 }
@@ -1682,13 +1677,7 @@ local_serve_kernel(const DevSim S, const LocalLoop A, ServeCtl* ctl, uint32_t se
 		}
 		if(!bar.join()) break;
 		if(blockIdx.x == 0) {
-			const uint32_t n = fired_ids_to_host(S, S.firedRing + (size_t) ring * S.W, hostIds);
-			__syncthreads();
-			if(threadIdx.x == 0) {
-				ctl->fired = n;
-				ctl->events = *(volatile unsigned long long*) &S.eventCount[ring];
-				st_release_sys(&ctl->done, want);
-			}
+			answer_request(S, ctl, ring, hostIds, want);
 		}
 	}
 	__syncthreads();
@@ -1853,13 +1842,7 @@ balanced_serve_kernel(const DevSim S, const LocalLoop A, ServeCtl* ctl, uint32_t
 		}
 		if(!bar.join()) break;
 		if(blockIdx.x == 0) {
-			const uint32_t n = fired_ids_to_host(S, S.firedRing + (size_t) ring * S.W, hostIds);
-			__syncthreads();
-			if(threadIdx.x == 0) {
-				ctl->fired = n;
-				ctl->events = *(volatile unsigned long long*) &S.eventCount[ring];
-				st_release_sys(&ctl->done, want);
-			}
+			answer_request(S, ctl, ring, hostIds, want);
 		}
 	}
 	__syncthreads();
@@ -2705,6 +2688,14 @@ void Simulation::init(const std::vector<const Network*>& nets, const Configurati
 		NB_CUDA(cudaStreamSynchronize(m_stream)); // host vectors go out of scope
 	}
 	S.ntypes = (uint32_t) m_types.size();
+	// the ids of one network as a table, where they are dense enough
+	if(!batch) {
+		const unsigned maxGid = *std::max_element(m_l2g.begin(), m_l2g.end());
+		if(maxGid < 4ull * N + 1024) {
+			m_g2lDense.assign((size_t) maxGid + 1, ~0u);
+			for(unsigned i = 0; i < N; ++i) m_g2lDense[m_l2g[i]] = i;
+		}
+	}
 
 	// synapses: the forward matrix, its delay groups and, with STDP, the
 	// reverse matrix of plastic synapses, built on the device where the
@@ -3159,6 +3150,10 @@ void Simulation::sync()
 unsigned Simulation::localIdx(unsigned g) const
 {
 	if(m_nets > 1) NB_THROW(NEMO_API_UNSUPPORTED, "per-neuron access is not available on a batch of networks");
+	if(!m_g2lDense.empty()) {
+		if(g >= m_g2lDense.size() || m_g2lDense[g] == ~0u) NB_THROW(NEMO_INVALID_INPUT, "Non-existing neuron index %u", g);
+		return m_g2lDense[g];
+	}
 	auto it = m_g2l[0].find(g);
 	if(it == m_g2l[0].end()) NB_THROW(NEMO_INVALID_INPUT, "Non-existing neuron index %u", g);
 	return it->second;
@@ -3697,6 +3692,9 @@ void Simulation::stepResident(uint32_t nf, uint32_t ni)
 {
 	volatile ServeCtl* c = reinterpret_cast<volatile ServeCtl*>(m_hServe);
 	const uint32_t want = m_serveSeq;
+	// no tag of the last round of sequence numbers may meet its own again
+	// (the loop is waiting: every word of its last answer has been read)
+	if(want == 1) for(uint32_t i = 0; i < SERVE_TAGGED; ++i) c->ids[i] = 0;
 	// a small firing stimulus goes in the request line itself
 	const bool inl = ni == 0 && nf <= SERVE_INLINE;
 	if(inl) {
@@ -3709,32 +3707,43 @@ void Simulation::stepResident(uint32_t nf, uint32_t ni)
 	std::atomic_thread_fence(std::memory_order_seq_cst);
 	if(!m_serving) launchServe();
 	const auto t0 = std::chrono::steady_clock::now();
-	for(uint32_t polls = 1;; ++polls) {
-		if(c->done == want) break;
-		if((polls & 63u) == 0) {
-			const cudaError_t q = cudaEventQuery(m_serveEnd);
-			if(q == cudaSuccess) {
-				if(c->done == want) break;
-				// the loop ended before this request: it was idle for too
-				// long (launch it again), or a grid barrier gave up
-				// (checkBarrier throws)
-				m_serving = false;
-				checkBarrier();
-				launchServe();
-			} else if(q != cudaErrorNotReady) {
-				NB_CUDA(q);
+	// spins until a word of the answer carries this request's tag
+	uint32_t polls = 0;
+	auto tagged = [&](volatile unsigned long long& word) -> uint32_t {
+		for(;;) {
+			const unsigned long long w = word;
+			if((uint32_t) (w >> 32) == want) return (uint32_t) w;
+			if((++polls & 63u) == 0) {
+				const cudaError_t q = cudaEventQuery(m_serveEnd);
+				if(q == cudaSuccess) {
+					if((uint32_t) (word >> 32) == want) continue;
+					// the loop ended before this request: it was idle for too
+					// long (launch it again), or a grid barrier gave up
+					// (checkBarrier throws)
+					m_serving = false;
+					checkBarrier();
+					launchServe();
+				} else if(q != cudaErrorNotReady) {
+					NB_CUDA(q);
+				}
+				if(std::chrono::steady_clock::now() - t0 > std::chrono::seconds(RESIDENT_REPLY_LIMIT_S)) {
+					NB_THROW(NEMO_CUDA_ERROR, "resident step loop: no reply within %u s", RESIDENT_REPLY_LIMIT_S);
+				}
 			}
-			if(std::chrono::steady_clock::now() - t0 > std::chrono::seconds(RESIDENT_REPLY_LIMIT_S)) {
-				NB_THROW(NEMO_CUDA_ERROR, "resident step loop: no reply within %u s", RESIDENT_REPLY_LIMIT_S);
-			}
-		}
 #if defined(__x86_64__)
-		__builtin_ia32_pause();
+			__builtin_ia32_pause();
 #endif
+		}
+	};
+	const uint32_t fired = tagged(c->reply[0]);
+	stepEvents += tagged(c->reply[1]);
+	if(fired <= SERVE_TAGGED) {
+		m_fired.resize(fired);
+		for(uint32_t i = 0; i < fired; ++i) m_fired[i] = tagged(c->ids[i]);
+	} else {
+		std::atomic_thread_fence(std::memory_order_seq_cst);
+		m_fired.assign(m_hFiredIds, m_hFiredIds + fired);
 	}
-	std::atomic_thread_fence(std::memory_order_seq_cst);
-	m_fired.assign(m_hFiredIds, m_hFiredIds + c->fired);
-	stepEvents += c->events;
 	m_serveSeq = serve_next(m_serveSeq);
 	m_cycle++;
 	m_timerSteps++;
@@ -3757,15 +3766,23 @@ const std::vector<unsigned>& Simulation::step(const unsigned* fstim, size_t nf,
 	std::vector<std::pair<uint32_t, float>>& cur = m_stepCurrents;
 	cur.clear();
 	if(ni) {
-		std::unordered_map<uint32_t, size_t> at;
+		// where a neuron's current stands in `cur`, valid for this call's stamp
+		if(m_curStamp.empty()) {
+			m_curStamp.assign(m_N, 0);
+			m_curAt.resize(m_N);
+		}
+		if(++m_curCall == 0) {
+			std::fill(m_curStamp.begin(), m_curStamp.end(), 0u);
+			m_curCall = 1;
+		}
 		for(size_t i = 0; i < ni; ++i) {
 			const uint32_t l = localIdx(inidx[i]);
-			auto it = at.find(l);
-			if(it == at.end()) {
-				at.emplace(l, cur.size());
+			if(m_curStamp[l] != m_curCall) {
+				m_curStamp[l] = m_curCall;
+				m_curAt[l] = (uint32_t) cur.size();
 				cur.emplace_back(l, icur[i]);
 			} else {
-				cur[it->second].second = icur[i];
+				cur[m_curAt[l]].second = icur[i];
 			}
 		}
 	}

@@ -44,7 +44,7 @@ constexpr uint32_t BARRIER_SPIN_LIMIT = 1u << 24;
 constexpr unsigned RESIDENT_REPLY_LIMIT_S = 20;
 
 // Requests to the resident step loop of nemo_step (mapped host memory):
-// the host writes the stimulus sizes and then go; the device writes done.
+// the host writes the request, the device the answer.
 // A request is two 8-byte words, each written and read whole: the
 // sequence number in the high half of both, the stimulus sizes (nf firing
 // indices, ni (index, current) pairs) in the low halves; it is complete
@@ -54,19 +54,21 @@ constexpr unsigned RESIDENT_REPLY_LIMIT_S = 20;
 // poll that finds the request also reads it: inl[i] = seq << 32 | local
 // index, each word checked by its sequence number as the request words
 // are, and req[0]'s low half is then SERVE_INLINE_FLAG | count.
+constexpr uint32_t SERVE_TAGGED = 4096;  // fired ids that an answer carries word by word
 constexpr uint32_t SERVE_INLINE = 6;
 constexpr uint32_t SERVE_INLINE_FLAG = 0x80000000u;
 struct ServeCtl {
 	unsigned long long req[2];
 	unsigned long long inl[SERVE_INLINE];
 	uint32_t pad0[16];
-	uint32_t done;     // sequence number of the last completed step
-	uint32_t fired;    // its fired neurons (global ids in the fired-id buffer)
-	unsigned long long events;  // its synaptic events
-	uint32_t pad1[28];
+	// the answer: sequence number << 32 | fired neurons, then | synaptic
+	// events, then (up to SERVE_TAGGED of them) | each fired global id
+	unsigned long long reply[2];
+	unsigned long long pad1[14];
+	unsigned long long ids[SERVE_TAGGED];
 };
 static_assert(offsetof(ServeCtl, inl) + 8 * SERVE_INLINE <= 64, "the request and its inline stimulus share one 64-byte line");
-static_assert(offsetof(ServeCtl, done) == 128, "the reply starts a line of its own");
+static_assert(offsetof(ServeCtl, reply) == 128, "the reply starts a line of its own");
 
 // STDP accumulation first tests a source against a shared-memory copy of the
 // "fired in the last 64 steps" bit-vector (W words), when it fits in this
@@ -450,6 +452,9 @@ private:
 	uint32_t* m_dFiredMapped = nullptr;
 	std::vector<uint32_t> m_stepScratch;
 	std::vector<std::pair<uint32_t, float>> m_stepCurrents;
+	std::vector<uint32_t> m_curStamp, m_curAt;  // per neuron: the last step() call that set its current, and where
+	uint32_t m_curCall = 0;
+	std::vector<uint32_t> m_g2lDense;  // one network: global id -> index (empty: ids too sparse, use m_g2l)
 	std::vector<unsigned> m_fired;
 	std::vector<uint32_t> m_outDegree;
 

@@ -36,6 +36,17 @@ def test_fire_stream(n, rate, stride, steps):
         assert np.array_equal(cp, co) and np.array_equal(ep, cp) and np.array_equal(ip, io)
 
 
+# an answer of one word of neurons or many, on both sides of the 4096 ids it
+# carries word by word
+@pytest.mark.parametrize("n,stride", [(1, 1), (33, 3), (1024, 1), (1025, 2), (4096, 1), (4097, 1), (9000, 2)])
+def test_step_answers(n, stride):
+    sp = nb.Simulation(firing_network(nb, n, 1.0, stride, 5), nb.Configuration())
+    so = O.Simulation(firing_network(O, n, 1.0, stride, 5), O.Configuration())
+    for _ in range(4):
+        assert list(sp.step()) == list(so.step())
+    assert sp.step_events() == 4 * n
+
+
 def test_fire_stream_longer_than_the_callers_buffer():
     sp = nb.Simulation(firing_network(nb, 100, 1.0, 1, 5), nb.Configuration())
     with pytest.raises(nb.NemoError):
