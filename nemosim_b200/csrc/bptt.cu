@@ -179,7 +179,7 @@ __device__ __forceinline__ void store_word(unsigned char* words, size_t i, int w
 // instruction issue (45k warp instructions per SM and ms, 12 us).
 constexpr int FWD_ROUNDS = 8;                        // mask loads in flight per lane
 constexpr int FWD_CHUNK = 32 * FWD_ROUNDS;           // synapses per pass over the lists
-constexpr int FWD_LIST = FWD_CHUNK / 4;              // entries of a compacted list
+constexpr int FWD_LIST = FWD_CHUNK / 4 + 4;          // entries of a compacted list (list 0 takes up to 3 more)
 constexpr int FWD_LISTS_BYTES = LOOP_THREADS / 32 * 4 * FWD_LIST * 4;
 
 // a synapse of the forward lists in shared memory (MODE 2: at most 65536
@@ -215,11 +215,14 @@ __device__ __noinline__ Real gather_counts(const BpttDev& D, const unsigned char
 	return (s[0] + s[2]) + (s[1] + s[3]);
 }
 
-// slot: t % D.ring, the place of ms t in the window; lists: this warp's four
-// lists of FWD_LIST entries (shared memory)
+// masks: all slices (global memory); window, slot: the last D.ring of them by
+// ms % D.ring and t % D.ring (MODE 2).  (Reading the newest slice from global
+// memory instead of waiting for its copy: 8.3 against 7.4 us a ms at
+// 4096 x 200 x 16.)  lists: this warp's four lists of FWD_LIST entries (shared
+// memory)
 template<typename Real, int MODE, typename Entry, typename Weight>
-__device__ __forceinline__ Real gather_masks(const BpttDev& D, const unsigned char* masks, int slot, int g,
-		const Entry* list, const Weight* w, int len, int t, unsigned* lists)
+__device__ __forceinline__ Real gather_masks(const BpttDev& D, const unsigned char* masks, const unsigned char* window, int slot,
+		int g, const Entry* list, const Weight* w, int len, int t, unsigned* lists)
 {
 	const unsigned FULL = 0xffffffffu;
 	const int lane = threadIdx.x & 31, laneLog = 31 - __clz(D.lanes);
@@ -229,30 +232,43 @@ __device__ __forceinline__ Real gather_masks(const BpttDev& D, const unsigned ch
 	auto mask_of = [&](int k) -> unsigned {
 		const int2 e = unpack_synapse(list[k]);
 		if(t < e.y) return 0u;
-		int at;
 		if(MODE == 2) {
-			at = slot - e.y;
+			int at = slot - e.y;
 			at += at < 0 ? D.ring : 0;
-			return load_mask(D, masks + (unsigned) (at * D.maskStride), e.x);
+			return load_mask(D, window + (unsigned) (at * D.maskStride), e.x);
 		}
-		at = (t - e.y) * D.groups + g;
+		const int at = (t - e.y) * D.groups + g;
 		return load_mask(D, masks + (size_t) (unsigned) at * D.maskStride, e.x);
 	};
 	Real s0 = Real(0), s1 = Real(0);
-	for(int base = 0; base < main; base += FWD_CHUNK) {
+	for(int base = 0; base < len; base += FWD_CHUNK) {
 		unsigned m[FWD_ROUNDS];
 #pragma unroll
 		for(int q = 0; q < FWD_ROUNDS; ++q) {
 			const int k = base + 32 * q + lane;
-			m[q] = k < main ? mask_of(k) : 0u;
+			m[q] = 0u;
+			if(base + 32 * q < len && k < len) m[q] = mask_of(k);
 		}
-		// lane l appends to list l % 4 (the entries k % 4 = l % 4)
+		// lane l appends to list l % 4 (the entries k % 4 = l % 4), the last
+		// len % 4 entries to list 0
 		int count = 0;
 #pragma unroll
 		for(int q = 0; q < FWD_ROUNDS; ++q) {
+			const int k0 = base + 32 * q;
+			if(k0 >= len) break;
+			const unsigned entry = (unsigned) (32 * q + lane) << 16 | m[q];
 			const unsigned live = __ballot_sync(FULL, m[q] != 0);
-			if(m[q]) lists[(lane & 3) * FWD_LIST + count + __popc(live & before)] = (unsigned) (32 * q + lane) << 16 | m[q];
-			count += __popc(live & mineBits);
+			if(k0 + 32 <= main) {
+				if(m[q]) lists[(lane & 3) * FWD_LIST + count + __popc(live & before)] = entry;
+				count += __popc(live & mineBits);
+			} else {
+				const unsigned tail = main > k0 ? FULL << (main - k0) : FULL;
+				const unsigned to0 = live & (0x11111111u | tail), mine = live & mineBits & ~tail, below = (1u << lane) - 1u;
+				const int count0 = __shfl_sync(FULL, count, 0);
+				if(to0 >> lane & 1u) lists[count0 + __popc(to0 & below)] = entry;
+				else if(m[q]) lists[(lane & 3) * FWD_LIST + count + __popc(mine & below)] = entry;
+				count += __popc((lane & 3) ? mine : to0);
+			}
 		}
 		__syncwarp();
 		const int n0 = __shfl_sync(FULL, count, sub & 3), n1 = __shfl_sync(FULL, count, (sub + 2) & 3);
@@ -276,12 +292,6 @@ __device__ __forceinline__ Real gather_masks(const BpttDev& D, const unsigned ch
 			}
 		}
 		__syncwarp();
-	}
-	if(sub == 0) {
-		for(int k = main; k < len; ++k) {
-			const Real wk = (Real) w[k];
-			if((mask_of(k) >> b) & 1u) s0 += wk;
-		}
 	}
 	if(subs == 2) s0 += s1;
 	else s0 += __shfl_xor_sync(FULL, s0, 2 * D.lanes);
@@ -383,6 +393,13 @@ __device__ __forceinline__ Trials<Real, V> gather_adjoint(const Real* now, bool 
 		return x;
 	};
 	if(valid) {
+		// the last len % 4 entries, one or two a sub-team
+		Trials<Real, V> rest[4 / SUBS];
+#pragma unroll
+		for(int h = 0; h < 4 / SUBS; ++h) {
+			const int k = 4 * groups + sub + h * SUBS;
+			if(k < len) rest[h] = load(off[k]);
+		}
 		int g = sub;
 		if(inside) {
 			for(; g + SUBS < groups; g += 2 * SUBS) {
@@ -412,8 +429,10 @@ __device__ __forceinline__ Trials<Real, V> gather_adjoint(const Real* now, bool 
 			add(x2, w[4 * g + 2]);
 			add(x3, w[4 * g + 3]);
 		}
-		if(sub == groups % SUBS) {
-			for(int k = 4 * groups; k < len; ++k) add(load(off[k]), w[k]);
+#pragma unroll
+		for(int h = 0; h < 4 / SUBS; ++h) {
+			const int k = 4 * groups + sub + h * SUBS;
+			if(k < len) add(rest[h], w[k]);
 		}
 	}
 #pragma unroll
@@ -452,6 +471,13 @@ __device__ __forceinline__ Trials<Real, V> gather_adjoint(const Real* now, bool 
 		sum.x[j] += __shfl_xor_sync(0xffffffffu, sum.x[j], lv);
 	}
 	return sum;
+}
+
+template<int BYTES>
+__device__ __forceinline__ void copy_async(void* to, const void* from)
+{
+	asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" :: "r"((unsigned) __cvta_generic_to_shared(to)), "l"(from),
+			"n"(BYTES) : "memory");
 }
 
 // one Euler sub-step and its reset; returns s
@@ -497,7 +523,7 @@ __global__ void __launch_bounds__(LOOP_THREADS, 1)
 bptt_forward_loop(const BpttDev D, const BpttState<Real> X, const BpttParams P, const LoopArgs L)
 {
 	extern __shared__ __align__(16) unsigned char raw[];
-	__shared__ int sAll, sMulti;
+	__shared__ int sAll;
 	const int gi = blockIdx.x / L.ctas, g = L.g0 + gi;
 	const int n0 = min(D.N, (int) (blockIdx.x % L.ctas) * L.cells), n1 = min(D.N, n0 + L.cells), nc = n1 - n0;
 	const int lanes = D.lanes, laneLog = 31 - __clz(lanes);
@@ -516,6 +542,7 @@ bptt_forward_loop(const BpttDev D, const BpttState<Real> X, const BpttParams P, 
 	Real* lossPart = r + cap;
 	const Entry* list;
 	const Weight* weight;
+	const int2* cells = nullptr;
 	unsigned char* window = nullptr;
 	__shared__ unsigned sLists[LOOP_THREADS / 32 * 4 * FWD_LIST];
 	unsigned* lists = sLists + (threadIdx.x >> 5) * 4 * FWD_LIST;
@@ -533,15 +560,26 @@ bptt_forward_loop(const BpttDev D, const BpttState<Real> X, const BpttParams P, 
 		}
 		list = se;
 		weight = sw;
-		window = raw + ((size_t) (reinterpret_cast<unsigned char*>(se + (last - first)) - raw) + 15) / 16 * 16;
+		// each neuron's place in the lists: read every ms, and L1 does not
+		// outlast a barrier
+		int2* sc = reinterpret_cast<int2*>(raw + ((size_t) (reinterpret_cast<unsigned char*>(se + (last - first)) - raw) + 7) / 8 * 8);
+		for(int cl = threadIdx.x; cl < nc; cl += LOOP_THREADS) {
+			const int beg = D.inStart[n0 + cl];
+			sc[cl] = make_int2(beg - first, D.inStart[n0 + cl + 1] - beg);
+		}
+		cells = sc;
+		window = raw + ((size_t) (reinterpret_cast<unsigned char*>(sc + nc) - raw) + 15) / 16 * 16;
 	}
+	auto place = [&](int cl) -> int2 {
+		if(MODE) return cells[cl];
+		const int beg = D.inStart[n0 + cl];
+		return make_int2(beg - first, D.inStart[n0 + cl + 1] - beg);
+	};
 	unsigned* counter = X.sync + sync_counter(gi, false, L.maxGroups);
 	const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 
-	if(tid == 0) {
-		sAll = 0;
-		sMulti = -D.ring - 1;  // the last ms in which a neuron fired more than once
-	}
+	if(tid == 0) sAll = 0;
+	int lastMulti = -D.ring - 1;  // the last ms in which a neuron of the group fired more than once
 	__syncthreads();
 	bool odd = false;
 	for(int k = tid; k < last - first; k += blockDim.x) odd |= !isfinite(weight[k]);
@@ -556,35 +594,40 @@ bptt_forward_loop(const BpttDev D, const BpttState<Real> X, const BpttParams P, 
 	// this thread's first item: its parameters, and its noise one ms ahead
 	const int myN = n0 + (tid >> laneLog), myB = b0 + (tid & (lanes - 1));
 	const bool mine = tid < items && (tid & (lanes - 1)) < nb;
-	float pa = 0, pb = 0, pc = 0, pd = 0, noise = 0;
+	float pa = 0, pb = 0, pc = 0, pd = 0, noise = 0, goal = 0;
+	auto ahead = [&](int t) {
+		noise = P.noise[((size_t) t * D.B + myB) * D.N + myN];
+		if(myN < D.R) goal = P.target[((size_t) t * D.B + myB) * D.R + myN];
+	};
 	if(mine) {
 		pa = P.a[myN];
 		pb = P.b[myN];
 		pc = P.c[myN];
 		pd = P.d[myN];
-		noise = P.noise[(size_t) myB * D.N + myN];
+		ahead(0);
 	}
 	__syncthreads();
 	const bool all = sAll != 0;
 
 	for(int t = 0; t < D.T; ++t) {
 		if(!SMOOTH) {
+			const int slot = t % D.ring;
 			if(t) {
 				const unsigned char* slice = X.masks + ((size_t) (t - 1) * D.groups + g) * D.maskStride;
+				const unsigned more = __ldcg(reinterpret_cast<const unsigned*>(slice));
 				if(MODE == 2) {
-					uint4* to = reinterpret_cast<uint4*>(window + (size_t) ((t - 1) % D.ring) * D.maskStride);
+					uint4* to = reinterpret_cast<uint4*>(window + (size_t) (slot ? slot - 1 : D.ring - 1) * D.maskStride);
 					const uint4* from = reinterpret_cast<const uint4*>(slice);
 					for(int k = tid; k < D.maskStride / 16; k += LOOP_THREADS) to[k] = __ldcg(from + k);
+					__syncthreads();
 				}
-				if(tid == 0 && __ldcg(reinterpret_cast<const unsigned*>(slice))) sMulti = t - 1;
-				__syncthreads();
+				if(more) lastMulti = t - 1;
 			}
-			const bool counts = all || t - sMulti <= D.ring;
-			const int slot = t % D.ring;
+			const bool counts = all || t - lastMulti <= D.ring;
 			for(int cl = warp; cl < nc; cl += LOOP_THREADS / 32) {
-				const int beg = D.inStart[n0 + cl] - first, len = D.inStart[n0 + cl + 1] - first - beg;
-				const Real s = counts ? gather_counts<Real>(D, X.words, g, list + beg, weight + beg, len, t)
-						: gather_masks<Real, MODE>(D, MODE == 2 ? window : X.masks, slot, g, list + beg, weight + beg, len, t, lists);
+				const int2 at = place(cl);
+				const Real s = counts ? gather_counts<Real>(D, X.words, g, list + at.x, weight + at.x, at.y, t)
+						: gather_masks<Real, MODE>(D, X.masks, window, slot, g, list + at.x, weight + at.x, at.y, t, lists);
 				if(lane < lanes) in[(cl << laneLog) + lane] = s;
 			}
 		} else {
@@ -592,8 +635,8 @@ bptt_forward_loop(const BpttDev D, const BpttState<Real> X, const BpttParams P, 
 			const int perWarp = 32 / team, cl0 = warp * perWarp + lane / team;
 			for(int cw = warp * perWarp, cl = cl0; cw < nc; cw += LOOP_THREADS / team, cl += LOOP_THREADS / team) {
 				const bool cell = cl < nc;
-				const int n = cell ? n0 + cl : n0;
-				const int beg = D.inStart[n] - first, len = cell ? D.inStart[n + 1] - first - beg : 0;
+				const int2 p = place(cell ? cl : 0);
+				const int beg = p.x, len = cell ? p.y : 0;
 				const bool valid = cell && b < nb;
 				const Real* at = X.S + b0 + b;
 				const Real s = lanes == BPTT_GROUP ? gather_dense<Real, 2, 8>(D, at, valid, list + beg, weight + beg, len, t, sub)
@@ -613,10 +656,9 @@ bptt_forward_loop(const BpttDev D, const BpttState<Real> X, const BpttParams P, 
 					pc = P.c[n];
 					pd = P.d[n];
 					noise = P.noise[((size_t) t * D.B + b) * D.N + n];
+					if(n < D.R) goal = P.target[((size_t) t * D.B + b) * D.R + n];
 				}
 				const size_t at = (size_t) n * D.B + b;
-				float goal = 0;
-				if(n < D.R) goal = P.target[((size_t) t * D.B + b) * D.R + n];
 				Real vi = v[i], ui = u[i];
 				if(t % D.ckpt == 0) {
 					const size_t k = (size_t) (t / D.ckpt) * NB + at;
@@ -665,11 +707,11 @@ bptt_forward_loop(const BpttDev D, const BpttState<Real> X, const BpttParams P, 
 				pd = P.d[myN];
 			}
 			if(L.ctas == 1) {
-				if(mine) noise = P.noise[((size_t) (t + 1) * D.B + myB) * D.N + myN];
+				if(mine) ahead(t + 1);
 				__syncthreads();
 			} else {
 				loop_arrive(counter);
-				if(mine) noise = P.noise[((size_t) (t + 1) * D.B + myB) * D.N + myN];
+				if(mine) ahead(t + 1);
 				if(!loop_wait(counter, L.base + (unsigned) (t + 1) * L.ctas, X.sync, X.hostError)) return;
 			}
 		}
@@ -736,9 +778,28 @@ bptt_backward_loop(const BpttDev D, const BpttState<Real> X, const BpttParams P,
 	Real* gA = lamR + cap;
 	Real* gB = gA + cap;
 	const int pad0 = D.outPad[n0];
-	Real* sw = reinterpret_cast<Real*>(raw + (6 * cap * sizeof(Real) + 15) / 16 * 16);
+	Real* sw = reinterpret_cast<Real*>(raw + ((11 * cap + 4 * (size_t) L.cells) * sizeof(Real) + 15) / 16 * 16);
 	unsigned* so = reinterpret_cast<unsigned*>(sw + (D.outPad[n1] - pad0));
+	// each neuron's two lists {start, entries}: read every ms, and L1 does not
+	// outlast a barrier
+	int4* sc = reinterpret_cast<int4*>(so + (D.outPad[n1] - pad0));
+	// a, b, c, d of each neuron, and the items' inputs of the coming ms (start
+	// state, input, trace, target), copied while the gathers run
+	Real* param = gB + cap;
+	Real* inV = param + 4 * L.cells;
+	Real* inU = inV + cap;
+	Real* inI = inU + cap;
+	Real* inR = inI + cap;
+	float* inT = reinterpret_cast<float*>(inR + cap);
 	if(SM) {
+		for(int cl = threadIdx.x; cl < nc; cl += LOOP_THREADS) {
+			const int n = n0 + cl, start = D.outStart[n], mid = D.outMid[n], beg = D.outPad[n] - pad0;
+			sc[cl] = make_int4(beg, mid - start, beg + (mid - start + 3) / 4 * 4, D.outStart[n + 1] - mid);
+			param[4 * cl] = (Real) P.a[n];
+			param[4 * cl + 1] = (Real) P.b[n];
+			param[4 * cl + 2] = (Real) P.c[n];
+			param[4 * cl + 3] = (Real) P.d[n];
+		}
 		for(int cl = threadIdx.x >> 5; cl < nc; cl += LOOP_THREADS / 32) {
 			const int n = n0 + cl, early = D.outMid[n] - D.outStart[n], to = D.outPad[n] - pad0;
 			const int gap = (early + 3) / 4 * 4 - early;
@@ -764,13 +825,11 @@ bptt_backward_loop(const BpttDev D, const BpttState<Real> X, const BpttParams P,
 		const bool inside = t + D.ring < D.T;
 		for(int cw = cw0, cl = cl0; cw < nc; cw += LOOP_THREADS / team, cl += LOOP_THREADS / team) {
 			const bool cell = cl < nc;
-			const int n = cell ? n0 + cl : n0;
-			const int start = D.outStart[n], mid = D.outMid[n];
-			const int len = !cell ? 0 : late ? D.outStart[n + 1] - mid : mid - start;
 			const bool valid = cell && tb < nb;
 			Trials<Real, V> s;
 			if(SM) {
-				const int beg = D.outPad[n] - pad0 + (late ? (mid - start + 3) / 4 * 4 : 0);
+				const int4 p = sc[cell ? cl : 0];
+				const int beg = late ? p.z : p.x, len = !cell ? 0 : late ? p.w : p.y;
 				const unsigned lim = (unsigned) min(limit, 0xffffffffull);
 				if(V == 1 && lv == BPTT_GROUP) {  // a warp holds two sub-teams of 16 lanes
 					s = gather_adjoint<Real, V, 2>(now, valid, inside, lim, so + beg, sw + beg, len, sub, lv);
@@ -778,6 +837,9 @@ bptt_backward_loop(const BpttDev D, const BpttState<Real> X, const BpttParams P,
 					s = gather_adjoint<Real, V, 4>(now, valid, inside, lim, so + beg, sw + beg, len, sub, lv);
 				}
 			} else {
+				const int n = cell ? n0 + cl : n0;
+				const int start = D.outStart[n], mid = D.outMid[n];
+				const int len = !cell ? 0 : late ? D.outStart[n + 1] - mid : mid - start;
 				const int beg = late ? mid : start;
 				if(V == 1 && lv == BPTT_GROUP) {
 					s = gather_adjoint<Real, V, 2>(now, valid, limit, D.outOff + beg, X.listW + beg, len, sub, lv);
@@ -819,27 +881,68 @@ bptt_backward_loop(const BpttDev D, const BpttState<Real> X, const BpttParams P,
 				}
 			}
 		}
+		__syncthreads();  // the copies below read what the replay stored
 		for(int t = t1 - 1; t >= t0; --t) {
+			if(SM) {
+				// each thread copies the inputs of its own items
+				for(int i = tid; i < items; i += LOOP_THREADS) {
+					const int bl = i & (lanes - 1), n = n0 + (i >> laneLog), b = b0 + bl;
+					if(bl >= nb) continue;
+					const size_t at = (size_t) n * D.B + b, s = (size_t) (t - t0) * NB + at;
+					copy_async<sizeof(Real)>(inV + i, X.segV + s);
+					copy_async<sizeof(Real)>(inU + i, X.segU + s);
+					copy_async<sizeof(Real)>(inI + i, X.I + (size_t) t * NB + at);
+					if(n < D.R) {
+						copy_async<sizeof(Real)>(inR + i, X.rHist + ((size_t) t * D.R + n) * D.B + b);
+						copy_async<4>(inT + i, P.target + ((size_t) t * D.B + b) * D.R + n);
+					}
+				}
+				asm volatile("cp.async.commit_group;" ::: "memory");
+			}
 			gather_all(t, false);
 			if(t + 1 < D.T) {
 				if(L.ctas == 1) __syncthreads();
 				else if(!loop_wait(counter, arrived, X.sync, X.hostError)) return;
 			}
 			gather_all(t, true);
+			if(SM) asm volatile("cp.async.wait_all;" ::: "memory");
 			__syncthreads();
 			for(int i = tid; i < items; i += LOOP_THREADS) {
 				const int bl = i & (lanes - 1), n = n0 + (i >> laneLog), b = b0 + bl;
 				if(bl >= nb) continue;
 				const size_t at = (size_t) n * D.B + b;
-				const size_t s = (size_t) (t - t0) * NB + at;
-				const Real v = X.segV[s], u = X.segU[s];
-				const Real I = __ldcs(X.I + (size_t) t * NB + at);
-				const Real a = P.a[n], bb = P.b[n], c = P.c[n], d = P.d[n];
+				Real v, u, I, a, bb, c, d, r = Real(0), goal = Real(0);
+				if(SM) {
+					const Real* p = param + 4 * (i >> laneLog);
+					v = inV[i];
+					u = inU[i];
+					I = inI[i];
+					a = p[0];
+					bb = p[1];
+					c = p[2];
+					d = p[3];
+					if(n < D.R) {
+						r = inR[i];
+						goal = (Real) inT[i];
+					}
+				} else {
+					const size_t s = (size_t) (t - t0) * NB + at;
+					v = X.segV[s];
+					u = X.segU[s];
+					I = __ldcs(X.I + (size_t) t * NB + at);
+					a = P.a[n];
+					bb = P.b[n];
+					c = P.c[n];
+					d = P.d[n];
+					if(n < D.R) {
+						r = X.rHist[((size_t) t * D.R + n) * D.B + b];
+						goal = (Real) P.target[((size_t) t * D.B + b) * D.R + n];
+					}
+				}
 				// dL/dS(t): readout trace and the inputs S(t) drives d ms later
 				Real lamS = Real(0);
 				if(n < D.R) {
-					const Real r = X.rHist[((size_t) t * D.R + n) * D.B + b];
-					const Real diff = r - (Real) P.target[((size_t) t * D.B + b) * D.R + n];
+					const Real diff = r - goal;
 					const Real lr = Real(2) * X.lossScale * diff + X.alpha * lamR[i];
 					lamR[i] = lr;
 					lamS = lr;
@@ -1071,7 +1174,7 @@ Bptt::Loop Bptt::planLoop(const std::vector<int>& start, int itemArrays, int min
 	const size_t items = (size_t) p.cells * D.lanes * itemArrays * realSize;
 	for(int mode = 2; mode > 0; --mode) {
 		if(!entry[mode]) continue;
-		const size_t bytes = longest * (entry[mode] + realSize) + items + 64 + (mode == 2 ? window : 0);
+		const size_t bytes = longest * (entry[mode] + realSize) + items + (size_t) p.cells * (16 + 4 * realSize) + 64 + (mode == 2 ? window : 0);
 		if(bytes <= m_limit) {
 			p.mode = mode;
 			p.smem = bytes;
@@ -1156,7 +1259,7 @@ Bptt::Bptt(unsigned N, unsigned B, unsigned T, unsigned R, unsigned ckpt, size_t
 		// offsets of the adjoint loop's shared lists are 32-bit
 		const bool narrow = (unsigned long long) NB * (D.ring + 1ull) <= 0xffffffffull;
 		const size_t bwdEntry[3] = { 0, narrow ? sizeof(unsigned) : 0, 0 };
-		m_bwd = planLoop(outPad, 6, BWD_MIN_CELLS, realSize, sms, bwdEntry, 0);
+		m_bwd = planLoop(outPad, 11, BWD_MIN_CELLS, realSize, sms, bwdEntry, 0);
 		m_maxGroups = sms;
 		BP_CUDA(cudaHostAlloc(&m_hostError, 4, cudaHostAllocMapped));
 		*m_hostError = 0;
