@@ -315,7 +315,7 @@ class Simulation:
         counts = np.zeros(max(steps, 1), np.uint32)
         events = np.zeros(max(steps, 1), np.uint64)
         cap = max_ids if max_ids is not None else steps * 4096
-        buf = np.zeros(max(cap, 1), np.uint32) if ids else None
+        buf = np.empty(max(cap, 1), np.uint32) if ids else None
         ln = C.c_size_t()
 
         def ptr(a):
@@ -324,7 +324,8 @@ class Simulation:
                                    cap if buf is not None else 0, C.byref(ln)))
         if buf is None:
             return counts[:steps], events[:steps], None
-        return counts[:steps], events[:steps], buf[: ln.value].copy()
+        buf.resize(ln.value, refcheck=False)  # in place: a copy of two million ids took 1.5 ms
+        return counts[:steps], events[:steps], buf
 
     def apply_stdp(self, reward: float):
         _check(lib().nemo_apply_stdp(self._h, float(reward)))
@@ -515,7 +516,7 @@ class Batch(Simulation):
         counts = np.zeros(max(steps, 1) * self.count, np.uint32)
         events = np.zeros(max(steps, 1), np.uint64)
         cap = max_ids if max_ids is not None else steps * 65536
-        buf = np.zeros(max(cap, 1), np.uint32) if ids else None
+        buf = np.empty(max(cap, 1), np.uint32) if ids else None
         ln = C.c_size_t()
 
         def ptr(a):
@@ -523,7 +524,9 @@ class Batch(Simulation):
         _check(lib().nemo_b200_run(self._h, steps, stdp_period, reward, ptr(counts), ptr(events), ptr(buf),
                                    cap if buf is not None else 0, C.byref(ln)))
         counts = counts[: steps * self.count].reshape(steps, self.count)
-        return counts, events[:steps], (buf[: ln.value].copy() if buf is not None else None)
+        if buf is not None:
+            buf.resize(ln.value, refcheck=False)
+        return counts, events[:steps], buf
 
     def streams(self, counts: np.ndarray, ids: np.ndarray):
         """Split a run's (counts, ids) into per-network (counts, ids)."""
