@@ -3220,7 +3220,7 @@ constexpr uint32_t LOCAL_MAX_IN = 320, LOCAL_MAX_IN_LARGE = 224, LOCAL_LARGE = 1
 // barriers 0.4 us at 1k to 20k neurons
 constexpr uint32_t BALANCED_MIN_THREADS = 512;
 // the fused step (planFused)
-constexpr uint32_t FUSED_MAX_OUT_LARGE = 640, FUSED_LARGE = 900000;
+constexpr uint32_t FUSED_MAX_OUT_LARGE = 1024, FUSED_LARGE = 900000;
 // One cluster of 16 CTAs up to this many neurons: 1000 x 100 takes 3.24 us a
 // step against 3.60 with the grid barrier, 2000 x 100 3.38 against 3.67,
 // 5000 x 100 3.81 against 3.79 (with STDP 5.10 against 4.73).
@@ -3559,7 +3559,12 @@ void Simulation::launchFused(unsigned n)
 // networks, delays to 20 ms):
 //   300k neurons, fan-out 100 12.9 / 17.9, 300 16.8 / 19.7, 600 24.8 / 23.8, 1000 37.4 / 30.4;
 //   with STDP 100 17.7 / 22.2, 300 27.4 / 25.4;
-//   960k neurons, 600 60.5 / 68.4;  with STDP 100 51.3 / 55.1, 600 101 / 85
+//   960k neurons, 600 60.5 / 68.4, 800 69.1 / 77.2, 1000 79.5 / 88.0;
+//   with STDP 100 51.3 / 55.1, 600 101 / 85
+//   1.92M neurons, 600 107 / 129, 1000 137 / 169
+// and 256 mixed networks (4.5M neurons, fan-out 100 to 1000) 262 / 325: with
+// enough warps to fill the SMs several times over, one warp's long list no
+// longer holds the others up.
 void Simulation::planFused()
 {
 	for(const HostType& t : m_types) if(t.desc.kind == KIND_KURAMOTO) return;
