@@ -284,12 +284,12 @@ NEMO_B200_API nemo_status_t nemo_b200_set_profiling(nemo_simulation_t, int on);
  * off. */
 NEMO_B200_API nemo_status_t nemo_b200_set_graphs(nemo_simulation_t, int on);
 /* Choose how nemo_b200_run advances the steps between applyStdp calls: one
- * persistent cooperative launch per segment, its update and delivery phases
- * separated by grid barriers (on), or two launches per step (off).  The
- * default is on, except for networks with more than two neurons per thread
- * of the persistent loop's co-resident CTAs (large batches), where one
- * launch per phase over the whole network is faster.  With it off, nemo_step
- * uses two launches per call.  Results are identical. */
+ * cooperative launch per segment (on), or one or two launches per step (off).
+ * The default is on, except for networks with more than two neurons per
+ * thread of the persistent loop's co-resident CTAs (large batches), where
+ * launches over the whole network are faster.  Which form of either runs
+ * follows from the network's size and degrees.  With it off, nemo_step uses
+ * two launches per call.  Results are identical. */
 NEMO_B200_API nemo_status_t nemo_b200_set_persistent(nemo_simulation_t, int on);
 /* nemo_step's resident step loop (no counterpart in the reference, whose
  * step runs on the host, src/nemo/cpu/Simulation.cpp:94-111): when the
