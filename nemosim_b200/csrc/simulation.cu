@@ -1855,11 +1855,18 @@ balanced_serve_kernel(const DevSim S, const LocalLoop A, ServeCtl* ctl, uint32_t
 // neurons' groups for the next step and accumulates STDP for its targets, so
 // a step needs neither work lists nor their reservations, and deliveries
 // overlap the updates of other warps: 24 networks of 400k neurons and 80M
-// synapses take 18.8 us a step, against 29.8 with deliver_kernel and
+// synapses take 18.1 us a step, against 29.8 with deliver_kernel and
 // update_kernel at two partitions per SM and 23.0 at one of 128 neurons per
-// CTA.  The noise comes from the libm tables (evaluated: 20.9).
+// CTA.  The noise comes from the libm tables (evaluated: 20.9 against 18.8 with tables).
 // deliver: not in the last step before applyStdp may run.
-__global__ void __launch_bounds__(FUSED_THREADS, 8)
+// CTAS: CTAs per SM.  Moderate degrees are bound by the latency of dependent
+// loads and want the warps: 10 (48 registers) against 8 (64) take 18.1 / 18.9
+// us a step there, 300k neurons x 100 12.6 / 12.9, with STDP 16.8 / 17.7 (12,
+// which spills, 20.0, 14.3 and 18.3; CTAs of 32, 64, 96 or 256 threads 19.4,
+// 18.0, 18.6 and 18.7 for the 24 networks).  Long lists want the loads in
+// flight: 1.92M neurons x 600 108.1 / 107.1.
+template<int CTAS>
+__global__ void __launch_bounds__(FUSED_THREADS, CTAS)
 fused_step_kernel(const DevSim S, uint32_t cur, uint32_t ring, uint32_t offset, int fromDev, int deliver)
 {
 	chain_wait_then_release();
@@ -3536,6 +3543,12 @@ void Simulation::launchSteps(unsigned n)
 	if(n) single(n);
 }
 
+// the instance of fused_step_kernel for a network's largest out-degree
+static auto fused_step_for(uint32_t maxOut)
+{
+	return maxOut > LOCAL_MAX_OUT ? fused_step_kernel<8> : fused_step_kernel<10>;
+}
+
 // n consecutive steps of fused_step_kernel, one launch each
 void Simulation::launchFused(unsigned n)
 {
@@ -3545,7 +3558,7 @@ void Simulation::launchFused(unsigned n)
 	timedEnd();
 	for(unsigned i = 0; i < n; ++i) {
 		timedBegin(K_STEP);
-		launch_chained(fused_step_kernel, grid, FUSED_THREADS, 0, m_stream, m_dev, (uint32_t) (m_cycle & 1),
+		launch_chained(fused_step_for(m_maxOutDeg), grid, FUSED_THREADS, 0, m_stream, m_dev, (uint32_t) (m_cycle & 1),
 				(uint32_t) (m_cycle % m_dev.R), 0u, 0, (int) (i + 1 < n));
 		timedEnd();
 		m_cycle++;
@@ -3557,8 +3570,8 @@ void Simulation::launchFused(unsigned n)
 // types, and degrees small enough for one warp beside the other work of a
 // step.  Microseconds a step, fused / two launches (batches of equal example
 // networks, delays to 20 ms):
-//   300k neurons, fan-out 100 12.9 / 17.9, 300 16.8 / 19.7, 600 24.8 / 23.8, 1000 37.4 / 30.4;
-//   with STDP 100 17.7 / 22.2, 300 27.4 / 25.4;
+//   300k neurons, fan-out 100 12.6 / 17.9, 300 16.8 / 19.7, 600 24.8 / 23.8, 1000 37.4 / 30.4;
+//   with STDP 100 16.8 / 22.2, 300 27.4 / 25.4;
 //   960k neurons, 600 60.5 / 68.4, 800 69.1 / 77.2, 1000 79.5 / 88.0;
 //   with STDP 100 51.3 / 55.1, 600 101 / 85
 //   1.92M neurons, 600 107 / 129, 1000 137 / 169
@@ -3590,7 +3603,7 @@ void Simulation::buildGraph()
 		const unsigned grid = (m_N + FUSED_THREADS - 1) / FUSED_THREADS;
 		launch_chained(fused_deliver_kernel, grid, FUSED_THREADS, 0, m_stream, m_dev, 0u, 1);
 		for(unsigned k = 0; k < GRAPH_STEPS; ++k) {
-			launch_chained(fused_step_kernel, grid, FUSED_THREADS, 0, m_stream, m_dev, 0u, 0u, k, 1, (int) (k + 1 < GRAPH_STEPS));
+			launch_chained(fused_step_for(m_maxOutDeg), grid, FUSED_THREADS, 0, m_stream, m_dev, 0u, 0u, k, 1, (int) (k + 1 < GRAPH_STEPS));
 		}
 	} else {
 		const unsigned grid = (m_N + m_P - 1) / m_P;
