@@ -2036,18 +2036,25 @@ static const void* serve_kernel_for(uint32_t threads)
 // warp's item after next and the runs of its next item are loaded while an
 // item is processed (at 5 CTAs of 256 threads per SM: 48 registers, no
 // spills), so an item's two dependent prologue loads are off its path.
-template<bool ALL>
+// SPLIT: an item's rounds of 128 entries are dealt to 2^applyShift warps,
+// which repeat its prologue.  A warp per item leaves a small network's GPU
+// idle: 1000 x 100 has 32 items of 20 rounds each.  Microseconds a call with
+// and without: 1000 x 100 8.7 / 31, 10007 x 100 12.7 / 34.5, 20000 x 1000
+// 85 / 130, 50021 x 500 92 / 108.  The networks with enough items keep the
+// instance without, whose loop is shorter: 100k x 1000 452 / 468.
+template<bool ALL, bool SPLIT>
 __global__ void __launch_bounds__(STEP_THREADS, 5)
 apply_kernel(const DevSim S, int32_t reward)
 {
 	const uint32_t FULL = 0xffffffffu;
 	const uint32_t lane = threadIdx.x & 31;
 	const uint32_t batches = S.W;  // words of 32 targets
-	const unsigned long long items = (unsigned long long) batches * S.applySlices;
+	const unsigned long long items = (unsigned long long) batches * S.applySlices << (SPLIT ? S.applyShift : 0);
 	const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
 	// lane's target of item ii (N: none)
 	auto target_of = [&](unsigned long long ii) -> uint32_t {
 		if(ii >= items) return S.N;
+		if(SPLIT) ii >>= S.applyShift;
 		const uint32_t kk = (uint32_t) (ii / batches);
 		const uint32_t w = (uint32_t) (ii - (unsigned long long) kk * batches);
 		const uint32_t t = w * 32 + lane;
@@ -2060,7 +2067,7 @@ apply_kernel(const DevSim S, int32_t reward)
 		lo = 0;
 		len = 0;
 		if(ii < items && t < S.N) {
-			const uint32_t kk = (uint32_t) (ii / batches);
+			const uint32_t kk = (uint32_t) ((SPLIT ? ii >> S.applyShift : ii) / batches);
 			const uint32_t* run = S.rcmSlice + (size_t) kk * S.N + t;
 			const uint32_t a = run[0];
 			lo = S.rcmPtr[t] + a;
@@ -2081,7 +2088,8 @@ apply_kernel(const DevSim S, int32_t reward)
 		const uint32_t tnn = target_of(i + 2ull * nw);
 		run_of(i + nw, tn, nlo, nlen);
 		tn = tnn;
-		for(uint32_t off = 0; off < total; off += 32 * APPLY_ILP) {
+		const uint32_t part = SPLIT ? (uint32_t) i & ((1u << S.applyShift) - 1) : 0;
+		for(uint32_t off = part * 32 * APPLY_ILP; off < total; off += 32 * APPLY_ILP << (SPLIT ? S.applyShift : 0)) {
 			unsigned long long e[APPLY_ILP];
 			int32_t acc[APPLY_ILP];
 			uint32_t fwd[APPLY_ILP];
@@ -3065,8 +3073,16 @@ void Simulation::init(const std::vector<const Network*>& nets, const Configurati
 	// order holds across the whole grid
 	{
 		int perSm = 0;
-		NB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, apply_kernel<false>, STEP_THREADS, 0));
+		NB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, apply_kernel<false, false>, STEP_THREADS, 0));
 		m_applyGrid = (unsigned) std::max(1, perSm) * (unsigned) m_sms;
+		// warps per item: until there are twice as many as fit at once, and
+		// each has a full round on average (as many as fit: 50021 x 500
+		// 101 us; four or eight times as many: 94, 96)
+		if(S.stdp) {
+			const uint64_t items = std::max<uint64_t>(1, (uint64_t) S.W * S.applySlices);
+			const uint64_t each = rcmPtr[N] / items, warps = (uint64_t) m_applyGrid * (STEP_THREADS / 32);
+			while(items << S.applyShift < 2 * warps && each >> (S.applyShift + 1) >= 32 * APPLY_ILP) ++S.applyShift;
+		}
 	}
 	// default shape of the two-launch step (set while the persistent loop is
 	// not yet configured): two partitions per SM
@@ -3869,11 +3885,10 @@ void Simulation::applyStdpDevice(int32_t R)
 	stopServe();
 	flushStdp();
 	timedBegin(K_APPLY);
-	if(!m_weightsClamped) {
-		apply_kernel<true><<<m_applyGrid, STEP_THREADS, 0, m_stream>>>(m_dev, R);
-	} else {
-		apply_kernel<false><<<m_applyGrid, STEP_THREADS, 0, m_stream>>>(m_dev, R);
-	}
+	const bool split = m_dev.applyShift > 0;
+	auto* kernel = m_weightsClamped ? (split ? apply_kernel<false, true> : apply_kernel<false, false>)
+			: split ? apply_kernel<true, true> : apply_kernel<true, false>;
+	kernel<<<m_applyGrid, STEP_THREADS, 0, m_stream>>>(m_dev, R);
 	timedEnd();
 	// updatedWeight's result always lies within the clamp range of its sign
 	// class, so after one full pass every plastic weight does, and only the

@@ -152,6 +152,7 @@ struct DevSim {
 	// least k x sliceLen ([applySlices + 1][N]; the last row is the in-degree)
 	const uint32_t* rcmSlice;
 	uint32_t applySlices, sliceLen;
+	uint32_t applyShift; // an item of applyStdp is shared by 2^applyShift warps
 	// reverse matrix of all synapses into the targets of a type that reads
 	// its sources (Kuramoto): per target, source | (delay - 1) << 26 and the
 	// weight as given
