@@ -2422,7 +2422,9 @@ nemo_status_t Simulation::stepNoAlloc(const unsigned* fstim, size_t nf, const un
 // ---------------------------------------------------------------------------
 // libm calibration tables on the device
 
-LibmCalib device_calibration(int device)
+// stream: the copies run on it and have ended when the call returns (a copy
+// from pageable memory may return with its last piece still under way)
+LibmCalib device_calibration(int device, cudaStream_t stream)
 {
 	static std::mutex mtx;
 	static std::unordered_map<int, LibmCalib> cache;
@@ -2436,18 +2438,19 @@ LibmCalib device_calibration(int device)
 	NB_CUDA(cudaMalloc(&dSin, t.sinFlip.size() * 4));
 	NB_CUDA(cudaMalloc(&dKey, (nexc + 1) * 4));
 	NB_CUDA(cudaMalloc(&dVal, (nexc + 1) * 4));
-	NB_CUDA(cudaMemcpy(dLog, t.logFlip.data(), t.logFlip.size() * 4, cudaMemcpyHostToDevice));
-	NB_CUDA(cudaMemcpy(dSin, t.sinFlip.data(), t.sinFlip.size() * 4, cudaMemcpyHostToDevice));
+	NB_CUDA(cudaMemcpyAsync(dLog, t.logFlip.data(), t.logFlip.size() * 4, cudaMemcpyHostToDevice, stream));
+	NB_CUDA(cudaMemcpyAsync(dSin, t.sinFlip.data(), t.sinFlip.size() * 4, cudaMemcpyHostToDevice, stream));
 	if(nexc) {
-		NB_CUDA(cudaMemcpy(dKey, t.excKey.data(), nexc * 4, cudaMemcpyHostToDevice));
-		NB_CUDA(cudaMemcpy(dVal, t.excVal.data(), nexc * 4, cudaMemcpyHostToDevice));
+		NB_CUDA(cudaMemcpyAsync(dKey, t.excKey.data(), nexc * 4, cudaMemcpyHostToDevice, stream));
+		NB_CUDA(cudaMemcpyAsync(dVal, t.excVal.data(), nexc * 4, cudaMemcpyHostToDevice, stream));
 	}
 	// the host libm's results at every reachable argument (67 MB + 336 MB)
 	float *dLogVal, *dSinVal;
 	NB_CUDA(cudaMalloc(&dLogVal, t.logVal.size() * 4));
 	NB_CUDA(cudaMalloc(&dSinVal, t.sinVal.size() * 4));
-	NB_CUDA(cudaMemcpy(dLogVal, t.logVal.data(), t.logVal.size() * 4, cudaMemcpyHostToDevice));
-	NB_CUDA(cudaMemcpy(dSinVal, t.sinVal.data(), t.sinVal.size() * 4, cudaMemcpyHostToDevice));
+	NB_CUDA(cudaMemcpyAsync(dLogVal, t.logVal.data(), t.logVal.size() * 4, cudaMemcpyHostToDevice, stream));
+	NB_CUDA(cudaMemcpyAsync(dSinVal, t.sinVal.data(), t.sinVal.size() * 4, cudaMemcpyHostToDevice, stream));
+	NB_CUDA(cudaStreamSynchronize(stream));
 	LibmCalib c;
 	c.logFlip = dLog;
 	c.sinFlip = dSin;
@@ -3011,7 +3014,9 @@ void Simulation::init(const std::vector<const Network*>& nets, const Configurati
 	S.curExt = dalloc<float>(N);
 	S.slot = dalloc<ulonglong2>(N);
 	S.l2g = dalloc<uint32_t>(N);
-	NB_CUDA(cudaMemcpy(S.l2g, m_l2g.data(), (size_t) N * 4, cudaMemcpyHostToDevice));
+	// on the stream, behind dalloc's zeros: the stream does not wait for the
+	// legacy one, so a plain copy could be overwritten by them
+	NB_CUDA(cudaMemcpyAsync(S.l2g, m_l2g.data(), (size_t) N * 4, cudaMemcpyHostToDevice, m_stream));
 	S.l2gIdentity = 1;
 	for(size_t i = 0; i < N; ++i) {
 		if(m_l2g[i] != i) {
@@ -3048,11 +3053,12 @@ void Simulation::init(const std::vector<const Network*>& nets, const Configurati
 		}
 		if(!identity) {
 			m_streamOrder = dalloc<uint32_t>(N);
-			NB_CUDA(cudaMemcpy(m_streamOrder, order.data(), (size_t) N * 4, cudaMemcpyHostToDevice));
+			NB_CUDA(cudaMemcpyAsync(m_streamOrder, order.data(), (size_t) N * 4, cudaMemcpyHostToDevice, m_stream));
 		}
 		m_streamNet = dalloc<uint32_t>(N);
-		NB_CUDA(cudaMemcpy(m_streamNet, netOf.data(), (size_t) N * 4, cudaMemcpyHostToDevice));
+		NB_CUDA(cudaMemcpyAsync(m_streamNet, netOf.data(), (size_t) N * 4, cudaMemcpyHostToDevice, m_stream));
 		m_netCounts = dalloc<uint32_t>((size_t) S.R * nets.size());
+		NB_CUDA(cudaStreamSynchronize(m_stream)); // the host vectors go out of scope
 	}
 	NB_CUDA(cudaHostAlloc(&m_hFiredMapped, (size_t) S.W * 4, cudaHostAllocMapped));
 	NB_CUDA(cudaHostGetDevicePointer(&m_dFiredMapped, m_hFiredMapped, 0));
@@ -3061,7 +3067,7 @@ void Simulation::init(const std::vector<const Network*>& nets, const Configurati
 	NB_CUDA(cudaHostGetDevicePointer(&m_dServe, m_hServe, 0));
 	NB_CUDA(cudaEventCreateWithFlags(&m_serveEnd, cudaEventDisableTiming));
 
-	if(needCalib) S.calib = device_calibration(m_device);
+	if(needCalib) S.calib = device_calibration(m_device, m_stream);
 	NB_CUDA(cudaDeviceGetAttribute(&m_sms, cudaDevAttrMultiProcessorCount, m_device));
 	// the two-launch pre-phase: as many CTAs as fit on the GPU at once
 	{

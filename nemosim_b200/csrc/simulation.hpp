@@ -472,6 +472,6 @@ private:
 
 // Device copies of the libm calibration tables (one per device, kept for
 // the life of the process).
-LibmCalib device_calibration(int device);
+LibmCalib device_calibration(int device, cudaStream_t stream);
 
 } // namespace nemo_b200
