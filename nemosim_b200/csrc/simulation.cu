@@ -3511,7 +3511,7 @@ void Simulation::checkBarrier()
 	NB_CUDA(cudaMemcpy(m_hBarrierError, &m_barrier->error, 4, cudaMemcpyDeviceToHost));
 	if(*m_hBarrierError) {
 		*m_hBarrierError = 0;
-		NB_CUDA(cudaMemset(m_barrier, 0, sizeof(GridBarrier)));
+		NB_CUDA(cudaMemsetAsync(m_barrier, 0, sizeof(GridBarrier), m_stream));
 		m_barrierBase = 0;
 		m_barrierStale = false;
 		NB_THROW(NEMO_CUDA_ERROR, "persistent step loop: a grid barrier wait timed out");

@@ -30,6 +30,13 @@ def test_no_upload_beside_the_stream(source):
     assert [c for c in calls(source, "cudaMemcpy") if "HostToDevice" in c] == []
 
 
+@pytest.mark.parametrize("source", ["simulation.cu", "construction.cu"])
+def test_no_zeros_beside_the_stream(source):
+    """The barrier of the step loops is cleared after a wait gave up, and the
+    next launch counts its arrivals in it."""
+    assert calls(source, "cudaMemset") == []
+
+
 @pytest.mark.gpu
 def test_id_tables_of_fresh_simulations():
     """1000 fresh rings with scattered ids: a table of zeros answers 0 for
