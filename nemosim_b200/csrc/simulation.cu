@@ -791,6 +791,12 @@ __device__ __forceinline__ unsigned long long ld_relaxed_sys_u64(const unsigned 
 	return v;
 }
 
+// a word that the host polls: written whole, once, in bounded time
+__device__ __forceinline__ void st_relaxed_sys_u64(unsigned long long* p, unsigned long long v)
+{
+	asm volatile("st.relaxed.sys.u64 [%0], %1;" :: "l"(p), "l"(v) : "memory");
+}
+
 // n words from device memory (just written by other CTAs: read from L2)
 // to host memory by the threads of one CTA, 16 bytes a thread where both
 // ends are 16-byte aligned
@@ -816,8 +822,8 @@ __device__ __forceinline__ void st_release(uint32_t* p, uint32_t v)
 // Simulation.cpp:200-208) and its synaptic events, by the threads of CTA 0.
 // Up to SERVE_TAGGED ids travel like an inline stimulus: every 8-byte word of
 // the answer carries the request's sequence number, and the host takes each
-// word as it arrives, so nothing waits until the writes have reached host
-// memory (a release at system scope took 1.4 to 1.9 us).  More ids go to
+// word as it arrives, in any order, so nothing waits until the writes have
+// reached host memory (a release at system scope took 1.4 to 1.9 us).  More ids go to
 // hostIds, published by such a release.
 __device__ void answer_request(const DevSim& S, ServeCtl* ctl, uint32_t ring, uint32_t* hostIds, uint32_t want)
 {
@@ -833,11 +839,11 @@ __device__ void answer_request(const DevSim& S, ServeCtl* ctl, uint32_t ring, ui
 			uint32_t bits = lane < S.W ? __ldcg(words + lane) : 0u;
 			const uint32_t n = __popc(bits), incl = warp_inclusive_scan(n);
 			uint32_t pos = incl - n;
-			for(; bits; bits &= bits - 1) ctl->ids[pos++] = tag | global_id(lane * 32 + __ffs(bits) - 1);
+			for(; bits; bits &= bits - 1) st_relaxed_sys_u64(&ctl->ids[pos++], tag | global_id(lane * 32 + __ffs(bits) - 1));
 			const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
 			if(lane == 0) {
-				ctl->reply[0] = tag | total;
-				ctl->reply[1] = tag | (uint32_t) events;
+				st_relaxed_sys_u64(&ctl->reply[0], tag | total);
+				st_relaxed_sys_u64(&ctl->reply[1], tag | (uint32_t) events);
 			}
 		}
 		return;
@@ -871,8 +877,8 @@ __device__ void answer_request(const DevSim& S, ServeCtl* ctl, uint32_t ring, ui
 	uint32_t pos = sWarp[warp] + incl - n;
 	if(total <= SERVE_TAGGED) {
 		if(t == 0) {
-			ctl->reply[0] = tag | total;
-			ctl->reply[1] = tag | (uint32_t) events;
+			st_relaxed_sys_u64(&ctl->reply[0], tag | total);
+			st_relaxed_sys_u64(&ctl->reply[1], tag | (uint32_t) events);
 		}
 #pragma unroll
 		for(uint32_t j = 0; j < WREG; ++j) {
@@ -882,7 +888,7 @@ __device__ void answer_request(const DevSim& S, ServeCtl* ctl, uint32_t ring, ui
 			for(uint32_t bits = __ldcg(words + w); bits; bits &= bits - 1) sIds[pos++] = w * 32 + __ffs(bits) - 1;
 		}
 		__syncthreads();
-		for(uint32_t i = t; i < total; i += T) ctl->ids[i] = tag | global_id(sIds[i]);
+		for(uint32_t i = t; i < total; i += T) st_relaxed_sys_u64(&ctl->ids[i], tag | global_id(sIds[i]));
 		return;
 	}
 	for(uint32_t w = w0; w < w1; ++w) {
@@ -892,7 +898,7 @@ __device__ void answer_request(const DevSim& S, ServeCtl* ctl, uint32_t ring, ui
 	copy_words_to_host(S.firedIds, hostIds, total);
 	__syncthreads();
 	if(t == 0) {
-		ctl->reply[1] = tag | (uint32_t) events;
+		st_relaxed_sys_u64(&ctl->reply[1], tag | (uint32_t) events);
 		// a release at system scope: the host that sees the word sees every
 		// store the CTA made before the __syncthreads
 		asm volatile("st.release.sys.u64 [%0], %1;" :: "l"(&ctl->reply[0]), "l"(tag | total) : "memory");
