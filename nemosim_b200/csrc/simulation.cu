@@ -1057,10 +1057,15 @@ serve_kernel(const DevSim S, uint32_t P, unsigned long long cycle0, GridBarrier*
 // another loop follows (Simulation::ensureLists).
 //
 // SYNC: how the CTAs wait for one another, and where the accumulators are.
-// 1: one cluster, an mbarrier in each CTA's shared memory at which every CTA's
-// arrival is signalled; the accumulators lie in the owner's shared memory, as
-// four 32-bit words: a weight w adds its low 16 bits to one word and w >> 16
-// to another (no carry to pass on, exact for up to 65536 arrivals a step).
+// 1: one cluster, two mbarriers in each CTA's shared memory at which every
+// CTA's arrivals are signalled, taken in turn: arrivals at different CTAs are
+// not ordered, so a CTA may pass a phase and arrive at a peer's next one
+// before a third CTA's arrival at that peer has landed, and a single mbarrier
+// would count it in the wrong phase.  (An arrival two phases ahead needs every
+// CTA to have passed the first.)  The accumulators lie in the owner's shared
+// memory, as four 32-bit words: a weight w adds its low 16 bits to one word
+// and w >> 16 to another (no carry to pass on, exact for up to 65536 arrivals
+// a step).
 // 2: the grid barrier above, accumulators in global memory as in the other
 // loops.  planLocal says which is taken when.
 constexpr uint32_t LOCAL_GROUPS = 128;  // groups of a warp's list at a time
@@ -1076,7 +1081,7 @@ struct LoopBarrier {
 	GridBarrier* gb;
 	uint32_t* target;            // SYNC 2 (shared)
 	uint32_t* ok;                // (shared)
-	unsigned long long* mbar;    // SYNC 1 (shared)
+	unsigned long long* mbar;    // SYNC 1: two mbarriers, taken in turn (shared)
 	uint32_t limit;
 	uint32_t phase = 0;
 
@@ -1087,11 +1092,14 @@ struct LoopBarrier {
 			*target = base;
 			*ok = 1;
 			if(SYNC == 1) {
-				const uint32_t a = (uint32_t) __cvta_generic_to_shared(mbar);
-				asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(a), "r"(gridDim.x) : "memory");
+				for(uint32_t k = 0; k < 2; ++k) {
+					const uint32_t a = (uint32_t) __cvta_generic_to_shared(mbar + k);
+					asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(a), "r"(gridDim.x) : "memory");
+				}
 				asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 			}
 		}
+		__syncwarp();
 		if(SYNC == 1) cluster_sync();
 		else __syncthreads();
 	}
@@ -1133,7 +1141,7 @@ struct LoopBarrier {
 			}
 		} else {
 			__syncwarp();
-			const uint32_t a = (uint32_t) __cvta_generic_to_shared(mbar);
+			const uint32_t a = (uint32_t) __cvta_generic_to_shared(mbar + (phase & 1u));
 			if(lane < gridDim.x) {
 				asm volatile("{\n\t.reg .b32 r;\n\tmapa.shared::cluster.u32 r, %0, %1;\n\t"
 						"mbarrier.arrive.release.cluster.shared::cluster.b64 _, [r];\n\t}" :: "r"(a), "r"(lane) : "memory");
@@ -1143,7 +1151,7 @@ struct LoopBarrier {
 				for(uint32_t polls = 0;;) {
 					uint32_t done;
 					asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
-							"selp.b32 %0, 1, 0, p;\n\t}" : "=r"(done) : "r"(a), "r"(phase & 1u) : "memory");
+							"selp.b32 %0, 1, 0, p;\n\t}" : "=r"(done) : "r"(a), "r"((phase >> 1) & 1u) : "memory");
 					if(done) break;
 					if(give_up(gb, polls, limit)) {
 						fail();
@@ -1601,11 +1609,11 @@ local_run_kernel(const DevSim S, const LocalLoop A)
 	extern __shared__ __align__(16) unsigned char raw[];
 	__shared__ LocalCounters sC[2];  // by step parity: one is emptied while the other fills
 	__shared__ uint32_t sTarget, sOk;
-	__shared__ unsigned long long sBar;
+	__shared__ unsigned long long sBar[2];
 	LocalNeuron L;
 	local_begin<SYNC>(S, A, raw, L);
 	if(threadIdx.x < 2) sC[threadIdx.x] = LocalCounters{ 0, 0, 0 };
-	LoopBarrier<SYNC> bar(A.gb, &sTarget, &sOk, &sBar, S.waitLimit, A.base);
+	LoopBarrier<SYNC> bar(A.gb, &sTarget, &sOk, sBar, S.waitLimit, A.base);
 	const bool worker = threadIdx.x < A.workers, last = threadIdx.x >= blockDim.x - 32;
 	bool target = false;
 	for(uint32_t k = 0; k < A.steps; ++k) {
@@ -1651,11 +1659,11 @@ local_serve_kernel(const DevSim S, const LocalLoop A, ServeCtl* ctl, uint32_t se
 	extern __shared__ __align__(16) unsigned char raw[];
 	__shared__ LocalCounters sC;
 	__shared__ uint32_t sTarget, sOk;
-	__shared__ unsigned long long sBar;
+	__shared__ unsigned long long sBar[2];
 	LocalNeuron L;
 	local_begin<SYNC>(S, A, raw, L);
 	if(threadIdx.x == 0) sC = LocalCounters{ 0, 0, 0 };
-	LoopBarrier<SYNC> bar(A.gb, &sTarget, &sOk, &sBar, S.waitLimit, 0);
+	LoopBarrier<SYNC> bar(A.gb, &sTarget, &sOk, sBar, S.waitLimit, 0);
 	const bool worker = threadIdx.x < A.workers, last = threadIdx.x >= blockDim.x - 32;
 	uint32_t want = seq0;
 	unsigned long long c = A.cycle0;
