@@ -1045,7 +1045,7 @@ serve_kernel(const DevSim S, uint32_t P, unsigned long long cycle0, GridBarrier*
 //    CTA that has passed it may deliver to the next step while others still
 //    read this one's sums: the accumulators alternate between two buffers.
 //    The STDP accumulation of step t runs while the barrier of t + 1
-//    completes; with delays of at least 1 it needs its sources' histories of
+//    completes; with delays of 1 to 63 it needs its sources' histories of
 //    step t - 1 only, which rotate over three buffers;
 //  - the last warp signals and awaits the barrier, and some warps before it
 //    draw the noise of the coming step all along (local_noise): on the worker
@@ -1494,7 +1494,7 @@ __device__ __forceinline__ void local_deliver(const DevSim& S, const LocalNeuron
 // STDP accumulation of this step over the incoming plastic synapses of the
 // warp's targets, as process_list<1>, with the histories `prev` of the step
 // before: shifted by one, they are this step's but for the newest bit, which
-// a delay of at least 1 shifts out
+// a delay of 1 to 63 shifts out (a delay of 64 shifts by 0: stdpNeedsNewest)
 __device__ __forceinline__ void local_stdp(const DevSim& S, const LocalNeuron& L, bool target, const uint64_t* prev)
 {
 	const uint32_t FULL = 0xffffffffu, lane = threadIdx.x & 31;
@@ -3273,7 +3273,7 @@ void Simulation::planLocal()
 {
 	for(const HostType& t : m_types) if(t.desc.kind == KIND_KURAMOTO) return;
 	if(!m_dev.dEnd16) return;
-	const bool balanced = m_maxOutDeg > LOCAL_MAX_OUT
+	const bool balanced = m_maxOutDeg > LOCAL_MAX_OUT || stdpNeedsNewest()
 			|| (m_dev.stdp && m_maxPlasticInDeg > (m_N <= LOCAL_LARGE ? LOCAL_MAX_IN : LOCAL_MAX_IN_LARGE));
 	// rows of delay-group ends an odd number of words apart (bank conflicts)
 	m_localStride = (m_dev.dStride + 1) / 2 * 2;
@@ -3618,7 +3618,7 @@ void Simulation::planFused()
 {
 	for(const HostType& t : m_types) if(t.desc.kind == KIND_KURAMOTO) return;
 	if(!m_dev.dEnd16 || m_maxOutDeg > (m_N >= FUSED_LARGE ? FUSED_MAX_OUT_LARGE : LOCAL_MAX_OUT)) return;
-	if(m_maxPlasticInDeg > LOCAL_MAX_IN_LARGE) return;
+	if(m_maxPlasticInDeg > LOCAL_MAX_IN_LARGE || stdpNeedsNewest()) return;
 	if(!m_dev.slot2) m_dev.slot2 = dalloc<ulonglong2>(2 * (size_t) m_N);
 	m_fusedOn = m_fusedFits = true;
 }

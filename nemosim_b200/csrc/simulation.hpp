@@ -364,6 +364,11 @@ private:
 	uint32_t m_localWorkers = 0, m_localT = 0, m_localGrid = 0, m_localStride = 0;
 	size_t m_localSmem = 0;
 	bool m_listsStale = false;  // its launches left the other loops' work lists behind
+	// STDP over a delay of 64 (which an empty post-fire part allows) reads the
+	// source's history unshifted, the spike of the same step included:
+	// process_list has it, local_stdp, with the histories of the step before,
+	// has not
+	bool stdpNeedsNewest() const { return m_dev.stdp && m_maxDelay == 64; }
 	void planLocal();
 	uint32_t maxInDegree();
 	LocalLoop localArgs(unsigned steps) const;
