@@ -1240,6 +1240,7 @@ Bptt::Bptt(unsigned N, unsigned B, unsigned T, unsigned R, unsigned ckpt, size_t
 		outSyn[q] = (int) e;
 	}
 	try {
+		BP_CUDA(cudaStreamCreateWithFlags(&m_filling, cudaStreamNonBlocking));
 		D.inStart = upload(inStart);
 		D.inSd = upload(inSd);
 		D.inSyn = upload(inSyn);
@@ -1265,6 +1266,11 @@ Bptt::Bptt(unsigned N, unsigned B, unsigned T, unsigned R, unsigned ckpt, size_t
 		*m_hostError = 0;
 		if(fp64) allocState(X64);
 		else allocState(X32);
+		// the first pass may come on any stream: its zeros (barrier counters
+		// among them) and lists are in place before the handle is out
+		BP_CUDA(cudaStreamSynchronize(m_filling));
+		BP_CUDA(cudaStreamDestroy(m_filling));
+		m_filling = nullptr;
 	} catch(...) {
 		release();
 		throw;
@@ -1343,6 +1349,8 @@ Bptt::~Bptt()
 
 void Bptt::release() noexcept
 {
+	if(m_filling) cudaStreamDestroy(m_filling);
+	m_filling = nullptr;
 	for(void* p : m_allocs) cudaFree(p);
 	m_allocs.clear();
 	if(m_hostError) cudaFreeHost(m_hostError);
@@ -1437,7 +1445,7 @@ void* Bptt::alloc(size_t bytes)
 		NB_THROW(NEMO_CUDA_MEMORY_ERROR, "failed to allocate %zu bytes of device memory", bytes);
 	}
 	m_allocs.push_back(p);
-	BP_CUDA(cudaMemset(p, 0, bytes));
+	BP_CUDA(cudaMemsetAsync(p, 0, bytes, m_filling));
 	return p;
 }
 
@@ -1449,7 +1457,7 @@ const V* Bptt::upload(const std::vector<V>& v)
 		NB_THROW(NEMO_CUDA_MEMORY_ERROR, "failed to allocate device memory");
 	}
 	m_allocs.push_back(p);
-	if(!v.empty()) BP_CUDA(cudaMemcpy(p, v.data(), v.size() * sizeof(V), cudaMemcpyHostToDevice));
+	if(!v.empty()) BP_CUDA(cudaMemcpyAsync(p, v.data(), v.size() * sizeof(V), cudaMemcpyHostToDevice, m_filling));
 	return static_cast<const V*>(p);
 }
 

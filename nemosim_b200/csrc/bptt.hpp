@@ -100,6 +100,7 @@ private:
 	int m_maxGroups = 1;   // trial groups of one launch at most
 	size_t m_limit = 0;    // dynamic shared memory of a loop's CTA at most
 	unsigned* m_hostError = nullptr;  // mapped pinned
+	cudaStream_t m_filling = nullptr; // of the constructor's zeros and uploads
 	int m_device = 0;
 	size_t m_M = 0;
 	std::vector<void*> m_allocs;

@@ -24,16 +24,17 @@ def calls(source, name):
     return [" ".join(m.split()) for m in re.findall(r"\b%s\s*\([^;]*;" % name, text)]
 
 
-@pytest.mark.parametrize("source", ["simulation.cu", "construction.cu"])
+@pytest.mark.parametrize("source", ["simulation.cu", "construction.cu", "bptt.cu"])
 def test_no_upload_beside_the_stream(source):
     assert calls(source, "cudaMemcpyAsync")
     assert [c for c in calls(source, "cudaMemcpy") if "HostToDevice" in c] == []
 
 
-@pytest.mark.parametrize("source", ["simulation.cu", "construction.cu"])
+@pytest.mark.parametrize("source", ["simulation.cu", "construction.cu", "bptt.cu"])
 def test_no_zeros_beside_the_stream(source):
     """The barrier of the step loops is cleared after a wait gave up, and the
-    next launch counts its arrivals in it."""
+    next launch counts its arrivals in it; the differentiable loops count from
+    the zeros of a new model, on whatever stream they are called."""
     assert calls(source, "cudaMemset") == []
 
 
@@ -71,3 +72,27 @@ def test_stream_order_of_fresh_batches():
         counts, _, ids = batch.run(3)
         assert counts.tolist() == counts0.tolist(), k
         assert ids.tolist() == ids0.tolist(), k
+
+
+@pytest.mark.gpu
+def test_first_pass_of_a_fresh_model_on_a_side_stream():
+    """100 fresh differentiable models, each called at once on a stream that
+    does not wait for the legacy one."""
+    import torch
+    from nemosim_b200.bptt import DifferentiableNetwork
+    net = DifferentiableNetwork.random(200, 20, seed=2)
+    gen = torch.Generator(device="cuda").manual_seed(1)
+    noise = 6.0 * torch.randn((40, 4, 200), generator=gen, device="cuda")
+    target = torch.zeros((40, 4, 32), device="cuda")
+    W, a, b = net.tensors("cuda")
+    torch.cuda.synchronize()
+    side, want = torch.cuda.Stream(), None
+    for k in range(100):
+        with torch.cuda.stream(side):
+            model = net.model(trials=4, ms=40, readout=32, checkpoint_ms=20)
+            loss = model.loss(W, a, b, noise, target)
+            got = [loss.detach(), *torch.autograd.grad(loss, (W, a, b))]
+            side.synchronize()
+        want = want or got
+        assert all(torch.equal(x, y) for x, y in zip(got, want)), k
+    assert float(want[0]) > 0 and float(want[1].abs().max()) > 0
