@@ -361,6 +361,12 @@ NEMO_B200_API nemo_status_t nemo_b200_run_stats(nemo_simulation_t, float* run_ms
  * persistent loop).  Results are identical for every shape. */
 NEMO_B200_API nemo_status_t nemo_b200_set_launch(nemo_simulation_t, unsigned partition, unsigned threads);
 NEMO_B200_API nemo_status_t nemo_b200_get_launch(nemo_simulation_t, unsigned* partition, unsigned* threads);
+/* The kernel that advances nemo_b200_run's steps as the simulation stands:
+ * local_run_kernel<1> (one cluster of CTAs), local_run_kernel<2>,
+ * balanced_run_kernel or run_kernel (cooperative launches of a segment), or
+ * fused_step_kernel or update_kernel (one or two launches per step).  The
+ * string is static. */
+NEMO_B200_API nemo_status_t nemo_b200_get_step_kernel(nemo_simulation_t, const char** name);
 /* Autotuner: times candidate launch shapes on `trial_steps` steps each,
  * starting every trial from a device-side snapshot of the simulation state
  * and restoring it afterwards (the simulation is left exactly as it was),

@@ -470,6 +470,12 @@ class Simulation:
         _check(lib().nemo_b200_get_launch(self._h, C.byref(p), C.byref(t)))
         return p.value, t.value
 
+    def step_kernel(self) -> str:
+        """The kernel that advances run()'s steps (an extension)."""
+        name = C.c_char_p()
+        _check(lib().nemo_b200_get_step_kernel(self._h, C.byref(name)))
+        return name.value.decode()
+
     def autotune(self, trial_steps: int = 50) -> float:
         """Pick the fastest launch shape on trial steps run from a snapshot
         (the simulation state is restored); returns microseconds per step."""

@@ -690,6 +690,12 @@ nemo_status_t nemo_b200_get_launch(nemo_simulation_t s, unsigned* partition, uns
 	});
 }
 
+nemo_status_t nemo_b200_get_step_kernel(nemo_simulation_t s, const char** name)
+{
+	NULLCHECK(s);
+	CALL(*name = S(s).stepKernel());
+}
+
 nemo_status_t nemo_b200_autotune(nemo_simulation_t s, unsigned trial_steps, float* us_per_step)
 {
 	NULLCHECK(s);

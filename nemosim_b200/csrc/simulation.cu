@@ -3420,6 +3420,14 @@ void Simulation::ensureLists() noexcept
 	publish_kernel<<<std::min(592u, (m_N + 255) / 256), 256, 0, m_stream>>>(m_dev, (uint32_t) ((m_cycle + 1) & 1));
 }
 
+const char* Simulation::stepKernel() const
+{
+	if(localActive()) {
+		return m_localSync == LOCAL_BALANCED ? "balanced_run_kernel" : m_localSync == 1 ? "local_run_kernel<1>" : "local_run_kernel<2>";
+	}
+	return persistentActive() ? "run_kernel" : m_fusedOn ? "fused_step_kernel" : "update_kernel";
+}
+
 void Simulation::setLaunch(uint32_t P, uint32_t T)
 {
 	stopServe();

@@ -1,0 +1,69 @@
+"""Which form of the step loop a network takes, on both sides of each rule,
+and that this form -- not another that stepped in for it -- gives the
+oracle's fire stream and its state, bit for bit."""
+import numpy as np
+import pytest
+
+import nemosim_b200 as nb
+import oracle as O
+from tests import nets
+from tests.test_single_barrier_gpu import conf, typed_network
+
+pytestmark = pytest.mark.gpu
+
+CLUSTER, GRID, BALANCED = "local_run_kernel<1>", "local_run_kernel<2>", "balanced_run_kernel"
+
+
+def same_bits(a, b):
+    """NaN for NaN, whatever its payload, and every other value by its bits."""
+    a, b = np.asarray(a, np.float32), np.asarray(b, np.float32)
+    return np.array_equal(np.where(np.isnan(a), np.float32(np.nan), a).view(np.uint32),
+                          np.where(np.isnan(b), np.float32(np.nan), b).view(np.uint32))
+
+
+def assert_same(sp, so, parts, steps, period, n):
+    cp, _, ip = sp.run(steps, period, 0.7, max_ids=steps * n + 1)
+    co, io = so.run(steps, period, 0.7, max_ids=steps * n + 1)
+    assert np.array_equal(cp, co) and np.array_equal(ip, io)
+    for t, ns in ((0, 2), (1, 4), (4, 2)):
+        if len(parts[t]):
+            assert same_bits(sp.type_state(t, ns, len(parts[t])), so.type_state(t, ns, len(parts[t])))
+
+
+# 2048 neurons | one cluster; out-degree 400 and, with STDP, a plastic
+# in-degree of 320 (224 beyond 12288 neurons and for one kernel per step):
+# the single barrier.  Largest plastic in-degrees of these networks, in turn:
+# 49, 292, 294, 415, 200, 234.
+@pytest.mark.parametrize("n,fanout,dmax,stdp,form,one_kernel", [
+    (1, 1, 1, False, CLUSTER, True), (2048, 40, 20, False, CLUSTER, True), (2049, 40, 20, False, GRID, True),
+    (700, 400, 20, False, CLUSTER, True), (700, 401, 20, False, BALANCED, False), (2048, 40, 20, True, CLUSTER, True),
+    (2500, 400, 20, True, GRID, False), (2500, 401, 20, True, BALANCED, False), (500, 600, 20, True, BALANCED, False),
+    (13000, 250, 10, True, GRID, True), (13000, 300, 10, True, BALANCED, False)])
+def test_form_and_results(n, fanout, dmax, stdp, form, one_kernel):
+    (pn, parts), (on, _) = typed_network(nb, n, fanout, dmax, 0.05, 6), typed_network(O, n, fanout, dmax, 0.05, 6)
+    sp, so = nb.Simulation(pn, conf(nb, stdp)), O.Simulation(on, conf(O, stdp))
+    assert sp.step_kernel() == form
+    assert_same(sp, so, parts, 60, 25 if stdp else 0, n)
+    assert sp.step_kernel() == form
+    sp.set_persistent(False)
+    assert sp.step_kernel() == ("fused_step_kernel" if one_kernel else "update_kernel")
+    assert_same(sp, so, parts, 30, 25 if stdp else 0, n)
+    sp.set_launch(64, 96)
+    assert sp.step_kernel() == "update_kernel"
+    sp.set_persistent(True)
+    assert sp.step_kernel() == form
+    sp.set_launch(64, 96)
+    assert sp.step_kernel() == "run_kernel"
+    assert_same(sp, so, parts, 30, 25 if stdp else 0, n)
+
+
+def test_types_beyond_the_forms():
+    net = nb.Network()
+    k = net.add_neuron_type("Kuramoto")
+    net.add_neuron(k, np.arange(40, dtype=np.uint32), np.float32(0.1), np.float32(0.0))
+    net.add_synapse(np.array([0], np.uint32), np.array([1], np.uint32), np.ones(1, np.uint32), np.full(1, 0.1, np.float32),
+                    np.zeros(1, np.uint8))
+    sim = nb.Simulation(net, nb.Configuration())
+    assert sim.step_kernel() == "run_kernel"
+    sim.set_persistent(False)
+    assert sim.step_kernel() == "update_kernel"
