@@ -358,7 +358,11 @@ NEMO_B200_API nemo_status_t nemo_b200_run_stats(nemo_simulation_t, float* run_ms
  * to a multiple of 32; at most 2048 for the two-launch step, where a CTA
  * owns one partition; a CTA of the persistent loop owns one or more) and
  * threads per CTA (a multiple of 32, at most 1024; 64 to 768 for the
- * persistent loop).  Results are identical for every shape. */
+ * persistent loop).  The shape that get_launch reports, set again, changes
+ * nothing.  Any other turns to the loop that takes a shape -- run_kernel, or
+ * two launches per step -- from the forms whose shape follows from the
+ * network (nemo_b200_get_step_kernel); the autotuner may choose those again.
+ * Results are identical for every shape. */
 NEMO_B200_API nemo_status_t nemo_b200_set_launch(nemo_simulation_t, unsigned partition, unsigned threads);
 NEMO_B200_API nemo_status_t nemo_b200_get_launch(nemo_simulation_t, unsigned* partition, unsigned* threads);
 /* The kernel that advances nemo_b200_run's steps as the simulation stands:

@@ -3108,7 +3108,7 @@ void Simulation::init(const std::vector<const Network*>& nets, const Configurati
 	// not yet configured): two partitions per SM
 	{
 		uint32_t P = (uint32_t) ((N + 2 * m_sms - 1) / (2 * m_sms));
-		setLaunch(P, std::min<uint32_t>(1024, std::max<uint32_t>(128, (P + 31) & ~31u)));
+		shapeLoop(P, std::min<uint32_t>(1024, std::max<uint32_t>(128, (P + 31) & ~31u)));
 	}
 	// the persistent step loop needs every CTA resident at once: a
 	// cooperative launch of at most the occupancy limit
@@ -3131,7 +3131,7 @@ void Simulation::init(const std::vector<const Network*>& nets, const Configurati
 			usePersistent = false;
 			// one neuron per thread in many small CTAs, against two
 			// partitions per SM: 23.0 / 29.8 us a step at 400k neurons
-			setLaunch(128, 128);
+			shapeLoop(128, 128);
 		}
 		if(m_runGrid) planLocal();
 	}
@@ -3428,7 +3428,14 @@ const char* Simulation::stepKernel() const
 	return persistentActive() ? "run_kernel" : m_fusedOn ? "fused_step_kernel" : "update_kernel";
 }
 
+// The shape in use, set again, keeps the form in use; another one goes to the
+// loop that has one.
 void Simulation::setLaunch(uint32_t P, uint32_t T)
+{
+	if(P != partition() || T != threads()) shapeLoop(P, T);
+}
+
+void Simulation::shapeLoop(uint32_t P, uint32_t T)
 {
 	stopServe();
 	if(persistentActive()) {
@@ -4148,7 +4155,7 @@ float Simulation::autotune(unsigned trialSteps)
 	try {
 		for(auto& c : cands) {
 			const bool local = c.first == 0;
-			if(!local) setLaunch(c.first, c.second);
+			if(!local) shapeLoop(c.first, c.second);
 			else if(pers) m_localOn = true;
 			else m_fusedOn = true;
 			auto own = [&](unsigned n) {
@@ -4191,7 +4198,7 @@ float Simulation::autotune(unsigned trialSteps)
 		restore();
 		sync();
 		for(void* b : backup) if(b) cudaFree(b);
-		setLaunch(P0, T0);
+		shapeLoop(P0, T0);
 		m_localOn = local0;
 		m_fusedOn = fused0;
 		profiling = prof;
@@ -4200,7 +4207,7 @@ float Simulation::autotune(unsigned trialSteps)
 	sync();
 	for(void* b : backup) if(b) cudaFree(b);
 	profiling = prof;
-	setLaunch(bestP, bestT);
+	shapeLoop(bestP, bestT);
 	m_localOn = pers ? bestLocal : local0;
 	m_fusedOn = pers ? fused0 : bestLocal;
 	return best * 1e3f / trialSteps;

@@ -257,6 +257,7 @@ public:
 	uint32_t partition() const { return localActive() ? m_localWorkers : persistentActive() ? m_runP : m_fusedOn ? FUSED_THREADS : m_P; }
 	uint32_t threads() const { return localActive() ? m_localT : persistentActive() ? m_runT : m_fusedOn ? FUSED_THREADS : m_T; }
 	void setLaunch(uint32_t P, uint32_t T);
+	void shapeLoop(uint32_t P, uint32_t T);
 	// the kernel that advances run()'s steps
 	const char* stepKernel() const;
 	bool persistentActive() const { return usePersistent && m_runGrid != 0; }

@@ -67,3 +67,23 @@ def test_types_beyond_the_forms():
     assert sim.step_kernel() == "run_kernel"
     sim.set_persistent(False)
     assert sim.step_kernel() == "update_kernel"
+
+
+@pytest.mark.parametrize("persistent", [True, False])
+@pytest.mark.parametrize("n,fanout", [(700, 40), (3000, 40), (700, 450)])
+def test_setting_the_reported_shape_changes_nothing(n, fanout, persistent):
+    a, b = (nb.Simulation(nb.example_random(n, fanout, 20, True), nets.standard_stdp(nb)) for _ in range(2))
+    for s in (a, b):
+        s.set_persistent(persistent)
+    form, shape = a.step_kernel(), a.launch()
+    a.set_launch(*shape)
+    assert (a.step_kernel(), a.launch()) == (form, shape) == (b.step_kernel(), b.launch())
+    ra, rb = a.run(130, 50, 1.0), b.run(130, 50, 1.0)
+    assert np.array_equal(ra[0], rb[0]) and np.array_equal(ra[2], rb[2])
+    a.set_launch(96, 192)
+    assert a.launch() == (96, 192) and a.step_kernel() == ("run_kernel" if persistent else "update_kernel")
+    a.set_launch(*a.launch())
+    assert a.launch() == (96, 192) and a.step_kernel() == ("run_kernel" if persistent else "update_kernel")
+    a.autotune(5)
+    ra, rb = a.run(130, 50, 1.0), b.run(130, 50, 1.0)
+    assert np.array_equal(ra[0], rb[0]) and np.array_equal(ra[2], rb[2])
