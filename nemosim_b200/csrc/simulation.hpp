@@ -39,7 +39,8 @@ static_assert(offsetof(GridBarrier, cmd) == 4, "one memset restarts count and cm
 constexpr uint32_t SERVE_STOP = 0x80000000u;
 __host__ __device__ inline uint32_t serve_next(uint32_t seq) { return seq == 0x7fffffffu ? 1u : seq + 1u; }
 constexpr unsigned RESIDENT_IDLE_MAX_US = 100000;  // the grid barrier's wait limit is far longer
-// polls of a grid-barrier or request wait before it gives up (seconds)
+// polls of a grid-barrier or request wait before it gives up (2.9 s at 171 ns
+// a poll, 3.4 s where a poll is followed by a pause)
 constexpr uint32_t BARRIER_SPIN_LIMIT = 1u << 24;
 constexpr unsigned RESIDENT_REPLY_LIMIT_S = 20;
 
