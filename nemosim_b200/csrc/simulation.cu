@@ -2714,7 +2714,16 @@ void Simulation::init(const std::vector<const Network*>& nets, const Configurati
 		ht.dState = dalloc<float>(state.size());
 		NB_CUDA(cudaMemcpyAsync(ht.dParam, param.data(), param.size() * 4, cudaMemcpyHostToDevice, m_stream));
 		NB_CUDA(cudaMemcpyAsync(ht.dState, state.data(), state.size() * 4, cudaMemcpyHostToDevice, m_stream));
-		if(kind == KIND_IZHIKEVICH) needCalib = true;
+		if(kind == KIND_IZHIKEVICH) {
+			needCalib = true;
+			// words of 32 neurons with a noisy one (sigma): a warp draws for
+			// the word whatever their number
+			for(unsigned i = 0, counted = ~0u; i < ht.n; ++i) {
+				if(param[(size_t) 4 * ht.n + i] == 0.0f || (l + i) / 32 == counted) continue;
+				counted = (l + i) / 32;
+				++m_noisyWords;
+			}
+		}
 		TypeRange& tr = S.types[m_types.size()];
 		tr.kind = kind;
 		tr.base = ht.base;
@@ -3265,6 +3274,18 @@ unsigned Simulation::runGridFor(uint32_t T) const
 // largest out-degree and one on the largest plastic in-degree.
 constexpr uint32_t LOCAL_MAX_OUT = 400;
 constexpr uint32_t LOCAL_MAX_IN = 320, LOCAL_MAX_IN_LARGE = 224, LOCAL_LARGE = 12288;
+// Draws of a noise warp in a step at most: with more worker warps there are
+// fewer noise warps beside them (7 from 769 neurons a CTA down to 1 at 960)
+// and the draws outlast the step.  Single-barrier / run_kernel at 4, 3, 2 and 1
+// noise warps (7, 9.3, 14.5 and 30 draws each; 125k, 130k, 135k and 142k
+// neurons): fan-out 100 9.0 / 15.1, 12.3 / 15.1, 17.7 / 15.2, 34.1 / 15.3 us a
+// step, with STDP 9.3 / 17.9, 12.5 / 17.6, 18.0 / 18.5 (135k); fan-out 300
+// 10.2 / 15.7, 12.4 / 15.8, 17.8 / 15.8, 34.5 / 15.9.  Balanced form, fan-out
+// 300 with STDP, at 4, 3 and 2: 17.8 / 19.5, 21.3 / 19.2, 26.6 / 20.0.  The
+// resident loop draws while it waits for the host: nemo_step takes 27.2 / 34.3
+// us a call at 135k neurons x 100, 43.0 / 34.8 at 142k; balanced 35.0 / 38.9 at
+// 125k, 38.6 / 39.6 and (fan-out 500) 37.3 / 36.7 at 130k.
+constexpr uint32_t LOCAL_MAX_DRAWS = 10, LOCAL_MAX_DRAWS_SERVED = 15, BALANCED_MAX_DRAWS = 7;
 // the balanced form's CTAs have at least this many threads, for its pre-phase:
 // 5k x 1000 with STDP 10.0 us a step, 12.0 with 128 threads; 1024 cost the
 // barriers 0.4 us at 1k to 20k neurons
@@ -3312,6 +3333,10 @@ void Simulation::planLocal()
 	auto plan = [&](int sync, uint32_t ctas) -> bool {
 		const uint32_t words = (m_dev.W + ctas - 1) / ctas, T = words * 32, grid = (m_dev.W + words - 1) / words;
 		if(threads(T) > LOCAL_THREADS || smem(sync, T) > LOCAL_SMEM_MAX) return false;
+		// words go round the CTAs, and so do the noisy ones
+		const uint32_t draws = (m_noisyWords + grid - 1) / grid, noiseWarps = (threads(T) - T) / 32 - 1;
+		if(draws > (balanced ? BALANCED_MAX_DRAWS : LOCAL_MAX_DRAWS_SERVED) * noiseWarps) return false;
+		m_localRuns = balanced || draws <= LOCAL_MAX_DRAWS * noiseWarps;
 		if(!fits(sync, T, grid)) {
 			cudaGetLastError();
 			return false;
@@ -3429,7 +3454,7 @@ void Simulation::ensureLists() noexcept
 
 const char* Simulation::stepKernel() const
 {
-	if(localActive()) {
+	if(localRuns()) {
 		return m_localSync == LOCAL_BALANCED ? "balanced_run_kernel" : m_localSync == 1 ? "local_run_kernel<1>" : "local_run_kernel<2>";
 	}
 	return persistentActive() ? "run_kernel" : m_fusedOn ? "fused_step_kernel" : "update_kernel";
@@ -3560,7 +3585,7 @@ void Simulation::checkBarrier()
 void Simulation::launchSteps(unsigned n)
 {
 	stopServe();
-	if(localActive()) {
+	if(localRuns()) {
 		launchLocal(n);
 		return;
 	}
@@ -4154,7 +4179,7 @@ float Simulation::autotune(unsigned trialSteps)
 	}
 	// the single-barrier loop or the fused step (their own shapes) against them
 	const bool fused0 = m_fusedOn;
-	if(pers ? m_localGrid != 0 : m_fusedFits) cands.emplace_back(0u, 0u);
+	if(pers ? m_localGrid != 0 && m_localRuns : m_fusedFits) cands.emplace_back(0u, 0u);
 	const uint32_t P0 = pers ? m_runP : m_P, T0 = pers ? m_runT : m_T;
 	float best = -1;
 	uint32_t bestP = P0, bestT = T0;
@@ -4215,7 +4240,7 @@ float Simulation::autotune(unsigned trialSteps)
 	for(void* b : backup) if(b) cudaFree(b);
 	profiling = prof;
 	shapeLoop(bestP, bestT);
-	m_localOn = pers ? bestLocal : local0;
+	m_localOn = pers && m_localRuns ? bestLocal : local0;
 	m_fusedOn = pers ? fused0 : bestLocal;
 	return best * 1e3f / trialSteps;
 }

@@ -255,8 +255,8 @@ public:
 	// launch shape of the active step loop (persistent or two-launch):
 	// partition size (neurons per partition; a CTA owns one or more) and
 	// threads per CTA; results do not depend on them
-	uint32_t partition() const { return localActive() ? m_localWorkers : persistentActive() ? m_runP : m_fusedOn ? FUSED_THREADS : m_P; }
-	uint32_t threads() const { return localActive() ? m_localT : persistentActive() ? m_runT : m_fusedOn ? FUSED_THREADS : m_T; }
+	uint32_t partition() const { return localRuns() ? m_localWorkers : persistentActive() ? m_runP : m_fusedOn ? FUSED_THREADS : m_P; }
+	uint32_t threads() const { return localRuns() ? m_localT : persistentActive() ? m_runT : m_fusedOn ? FUSED_THREADS : m_T; }
 	void setLaunch(uint32_t P, uint32_t T);
 	void shapeLoop(uint32_t P, uint32_t T);
 	// the kernel that advances run()'s steps
@@ -264,6 +264,8 @@ public:
 	bool persistentActive() const { return usePersistent && m_runGrid != 0; }
 	// the persistent loop's steps run through its single-barrier form
 	bool localActive() const { return persistentActive() && m_localOn; }
+	// those of run(), not only those of nemo_step
+	bool localRuns() const { return localActive() && m_localRuns; }
 	// step() keeps the persistent loop resident on the GPU between calls
 	// (serve_kernel) and ends it after this many microseconds without a
 	// call (at most RESIDENT_IDLE_MAX_US); 0: two kernel launches per step
@@ -363,7 +365,7 @@ private:
 	unsigned runGridFor(uint32_t T) const;
 	// the single-barrier loop: whether it is in use, its CTAs' way to wait
 	// (LoopBarrier), neurons and threads per CTA, CTAs, shared memory, row stride
-	bool m_localOn = false;
+	bool m_localOn = false, m_localRuns = false;
 	int m_localSync = 2;
 	uint32_t m_localWorkers = 0, m_localT = 0, m_localGrid = 0, m_localStride = 0;
 	size_t m_localSmem = 0;
@@ -413,6 +415,7 @@ private:
 	unsigned m_applyGrid = 1184;    // CTAs of apply_kernel
 	uint32_t m_P = 256, m_T = 256;
 	uint32_t m_maxOutDeg = 0, m_maxPlasticInDeg = 0;
+	uint32_t m_noisyWords = 0;  // words of 32 neurons with an Izhikevich neuron that has input noise at construction
 	int m_sms = 148;
 	void applyStdpDevice(int32_t fxReward);
 	void sync();

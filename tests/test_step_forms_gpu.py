@@ -87,3 +87,40 @@ def test_setting_the_reported_shape_changes_nothing(n, fanout, persistent):
     a.autotune(5)
     ra, rb = a.run(130, 50, 1.0), b.run(130, 50, 1.0)
     assert np.array_equal(ra[0], rb[0]) and np.array_equal(ra[2], rb[2])
+
+
+def noisy_network(n, noisy, hub):
+    """n Izhikevich neurons, the first `noisy` with input noise, three synapses
+    each and, with a hub, one of out-degree 401 (the balanced form)."""
+    net = nb.Network()
+    sigma = np.where(np.arange(n) < noisy, 6.0, 0.0).astype(np.float32)
+    ids = np.arange(n, dtype=np.uint32)
+    net.add_neuron(net.add_neuron_type("Izhikevich"), ids, *nets.exc_neuron_args(0.0)[:4], sigma, -13.0, -65.0)
+    rng = np.random.default_rng(n)
+    src = np.concatenate([np.repeat(ids, 3), np.full(398 if hub else 0, 5)]).astype(np.uint32)
+    net.add_synapse(src, rng.integers(0, n, len(src)).astype(np.uint32), rng.integers(1, 21, len(src)).astype(np.uint32),
+                    np.full(len(src), 4.0, np.float32), np.zeros(len(src), np.uint8))
+    return net
+
+
+# words of 32 neurons per CTA, neurons beyond, the noisy share; 27, 28, 29 and
+# 30 worker warps leave 4, 3, 2 and 1 warps for the noise (a word of 32 neurons
+# costs a draw when one of them is noisy)
+@pytest.mark.parametrize("words,more,noisy,hub,form", [
+    (28, 0, 1.0, False, GRID), (28, 1, 1.0, False, "run_kernel"), (28, 1, 0.5, False, GRID), (30, 0, 0.25, False, GRID),
+    (30, 0, 0.5, False, "run_kernel"), (30, 0, 0.0, False, GRID), (27, 0, 1.0, True, BALANCED), (27, 1, 1.0, True, "run_kernel"),
+    (27, 1, 0.5, True, BALANCED)])
+def test_noise_limit(words, more, noisy, hub, form):
+    import torch
+    n = words * 32 * torch.cuda.get_device_properties(0).multi_processor_count + more
+    a, b = (nb.Simulation(noisy_network(n, int(noisy * n), hub), nb.Configuration()) for _ in range(2))
+    assert a.step_kernel() == form
+    b.set_persistent(False)
+    b.set_launch(256, 256)
+    for steps in (1, 60):
+        ra, rb = a.run(steps, max_ids=steps * n), b.run(steps, max_ids=steps * n)
+        assert np.array_equal(ra[0], rb[0]) and np.array_equal(ra[2], rb[2])
+        # served by the same form up to 29 worker warps
+        assert [list(a.step([k])) for k in range(10)] == [list(b.step([k])) for k in range(10)]
+    assert noisy == 0 or ra[0].sum() > 0
+    assert same_bits(a.type_state(0, 2, n), b.type_state(0, 2, n))
