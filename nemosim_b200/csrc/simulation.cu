@@ -3582,10 +3582,20 @@ void Simulation::checkBarrier()
 // n consecutive steps: the persistent step loop, or whole CUDA graphs of
 // GRAPH_STEPS two-launch steps (captured once per launch shape and replayed
 // from a device cycle counter) and single launches for the rest
-void Simulation::launchSteps(unsigned n)
+// only: nothing else is launched in the call, whose time is then the launch's
+// latency.
+void Simulation::launchSteps(unsigned n, bool only)
 {
 	stopServe();
-	if(localRuns()) {
+	// The balanced form loads and stores its neurons once a launch: few steps
+	// of many neurons are faster in run_kernel or, a single one, as two
+	// launches.  Microseconds a call of 1, 2, 3, 4 and 6 steps, balanced /
+	// those: 100k x 1000 with STDP 62.7 / 53.5, 83.6 / 80.0, 102.7 / 100.3,
+	// 122.6 / 121.2, 162.1 / 162.2; 50k x 500 48.4 / 44.1, 57.6 / 56.9, 65.9 /
+	// 67.1; 20k x 1000 with STDP 51.9 / 46.5, 64.7 / 65.0.  A step per reward
+	// in a run of 100: 100k 63.7 / 61.3, 20k 33.6 / 37.6.
+	const bool brief = m_localSync == LOCAL_BALANCED && (n * 20000ull < m_N || (n == 1 && only));
+	if(localRuns() && !brief) {
 		launchLocal(n);
 		return;
 	}
@@ -4014,7 +4024,7 @@ void Simulation::run(unsigned steps, unsigned stdpPeriod, float reward, unsigned
 		for(unsigned i = 0; i < chunk;) {
 			const unsigned untilApply = stdpPeriod ? stdpPeriod - (done + i) % stdpPeriod : chunk - i;
 			const unsigned seg = std::min(chunk - i, untilApply);
-			launchSteps(seg);
+			launchSteps(seg, steps == 1);
 			i += seg;
 			if(stdpPeriod && (done + i) % stdpPeriod == 0) applyStdpDevice(R);
 		}

@@ -338,7 +338,7 @@ private:
 	void ensureQueryTables();
 	void freeKept() noexcept;
 	void launchStep(bool fullRecord);
-	void launchSteps(unsigned n);
+	void launchSteps(unsigned n, bool only);
 	void launchRun(unsigned n, bool finalStdp = true, const uint32_t* stim = nullptr, uint32_t nf = 0, uint32_t ni = 0,
 			uint32_t* hostFired = nullptr);
 	uint64_t m_barrierBase = 0;  // the barrier counter's value after the launches so far

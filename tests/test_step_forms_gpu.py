@@ -124,3 +124,20 @@ def test_noise_limit(words, more, noisy, hub, form):
         assert [list(a.step([k])) for k in range(10)] == [list(b.step([k])) for k in range(10)]
     assert noisy == 0 or ra[0].sum() > 0
     assert same_bits(a.type_state(0, 2, n), b.type_state(0, 2, n))
+
+
+@pytest.mark.parametrize("n,fanout", [(700, 450), (20_001, 420), (40_001, 420)])
+def test_brief_runs_of_the_balanced_form(n, fanout):
+    """Segments on both sides of the length from which the balanced form pays
+    (one step per 20000 neurons, two at least), one after the other."""
+    a, b = (nb.Simulation(nb.example_random(n, fanout, 20, True), nets.standard_stdp(nb)) for _ in range(2))
+    assert a.step_kernel() == BALANCED
+    b.set_launch(256, 384)
+    assert b.step_kernel() == "run_kernel"
+    for steps, period in ((60, 0), (1, 0), (1, 1), (2, 0), (3, 1), (1, 0), (12, 2), (3, 0), (15, 4), (40, 0)):
+        ra, rb = a.run(steps, period, 0.5, max_ids=steps * n), b.run(steps, period, 0.5, max_ids=steps * n)
+        assert np.array_equal(ra[0], rb[0]) and np.array_equal(ra[1], rb[1]) and np.array_equal(ra[2], rb[2])
+        assert list(a.step([5])) == list(b.step([5]))
+    assert ra[0].sum() > 0
+    assert same_bits(a.type_state(0, 2, n), b.type_state(0, 2, n))
+    assert np.array_equal(a.weights_fx(n * fanout), b.weights_fx(n * fanout))
