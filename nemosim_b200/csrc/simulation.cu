@@ -3753,7 +3753,14 @@ void Simulation::launchServe()
 		NB_CUDA(cudaHostGetDevicePointer(&m_dFiredIdsMapped, m_hFiredIds, 0));
 	}
 	// the barrier counter and the request word (count and cmd, adjacent)
-	const bool local = localActive();
+	// After a launch that served one step (a query, a reward or a pause follows
+	// each) the balanced form gives way to serve_kernel, whose launch loads no
+	// neurons.  Microseconds of a step and a set_neuron_state, balanced /
+	// serve_kernel: 100k x 300 with STDP 54.0 / 50.1, 50k x 500 45.0 / 43.4, 20k x
+	// 1000 45.1 / 44.1; with an applyStdp 100k x 1000 97.2 / 93.7.  From three
+	// steps a launch the balanced form is ahead (187 / 192).
+	const bool local = localActive() && !(m_localSync == LOCAL_BALANCED && m_served == 1);
+	m_served = 0;
 	if(local && m_localSync != LOCAL_BALANCED) flushStdp();  // of a step of another loop
 	else ensureLists();
 	NB_CUDA(cudaMemsetAsync(&m_barrier->count, 0, 8, m_stream));
@@ -3856,6 +3863,7 @@ void Simulation::stepResident(uint32_t nf, uint32_t ni)
 		m_fired.assign(m_hFiredIds, m_hFiredIds + fired);
 	}
 	m_serveSeq = serve_next(m_serveSeq);
+	++m_served;
 	m_cycle++;
 	m_timerSteps++;
 	// the single-barrier loop accumulates before it ends

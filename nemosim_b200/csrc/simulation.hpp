@@ -369,6 +369,7 @@ private:
 	int m_localSync = 2;
 	uint32_t m_localWorkers = 0, m_localT = 0, m_localGrid = 0, m_localStride = 0;
 	size_t m_localSmem = 0;
+	uint64_t m_served = 0;      // steps of the resident loop's last launch
 	bool m_listsStale = false;  // its launches left the other loops' work lists behind
 	// STDP over a delay of 64 (which an empty post-fire part allows) reads the
 	// source's history unshifted, the spike of the same step included:

@@ -141,3 +141,23 @@ def test_brief_runs_of_the_balanced_form(n, fanout):
     assert ra[0].sum() > 0
     assert same_bits(a.type_state(0, 2, n), b.type_state(0, 2, n))
     assert np.array_equal(a.weights_fx(n * fanout), b.weights_fx(n * fanout))
+
+
+def test_resident_launches_of_one_step():
+    """The balanced form gives way to the persistent loop after launches that
+    served one step, and returns after one that served more."""
+    n, fanout = 900, 430
+    a, b = (nb.Simulation(nb.example_random(n, fanout, 20, True), nets.standard_stdp(nb)) for _ in range(2))
+    assert a.step_kernel() == BALANCED
+    b.set_resident_step(0)
+    for length in (1, 1, 1, 5, 1, 1, 30, 2, 1, 1, 1, 7):
+        for k in range(length):
+            f, i = [k, 3 * k + 1], [(n - 1 - k, 12.0)] if k % 2 else None
+            assert list(a.step(f, i)) == list(b.step(f, i))
+        for s in (a, b):
+            s.apply_stdp(0.5)
+            s.set_neuron_state(7, 0, -12.0)
+        ra, rb = a.run(2, max_ids=2 * n), b.run(2, max_ids=2 * n)
+        assert np.array_equal(ra[2], rb[2])
+    assert same_bits(a.type_state(0, 2, n), b.type_state(0, 2, n))
+    assert np.array_equal(a.weights_fx(n * fanout), b.weights_fx(n * fanout))
