@@ -369,7 +369,9 @@ NEMO_B200_API nemo_status_t nemo_b200_get_launch(nemo_simulation_t, unsigned* pa
  * local_run_kernel<1> (one cluster of CTAs), local_run_kernel<2>,
  * balanced_run_kernel or run_kernel (cooperative launches of a segment), or
  * fused_step_kernel or update_kernel (one or two launches per step).  The
- * string is static. */
+ * local_ forms stand back for run_kernel while the network fires often, and
+ * balanced_run_kernel leaves runs of a few steps to it.  The string is
+ * static. */
 NEMO_B200_API nemo_status_t nemo_b200_get_step_kernel(nemo_simulation_t, const char** name);
 /* Autotuner: times candidate launch shapes on `trial_steps` steps each,
  * starting every trial from a device-side snapshot of the simulation state

@@ -1540,10 +1540,14 @@ __device__ __forceinline__ void local_stdp(const DevSim& S, const LocalNeuron& L
 
 // Update of step c (ring row ring) for this thread's neuron; returns whether it
 // is an STDP target of this step.  slot (SYNC 2), hist: this step's
-// accumulators and, with STDP, its histories.
+// accumulators and, with STDP, its histories.  load: each warp's entries so
+// far (shared; null: not counted), the synapses of its spikes and its STDP
+// entries, for Simulation::noteLoad.  (Counted here, where the sums are at
+// hand: a count in or beside local_deliver changed that loop's code and made
+// the cluster's step 3.4 to 4.3 us instead of 3.2 to 3.7.)
 template<int SYNC, bool STIM>
 __device__ __forceinline__ bool local_update(const DevSim& S, LocalNeuron& L, ulonglong2* slot, uint64_t* hist,
-		unsigned long long c, uint32_t ring, LocalCounters& C)
+		unsigned long long c, uint32_t ring, LocalCounters& C, uint32_t* load)
 {
 	const uint32_t lane = threadIdx.x & 31, buf = (uint32_t) (c & 1);
 	bool fired = false, target = false;
@@ -1594,6 +1598,7 @@ __device__ __forceinline__ bool local_update(const DevSim& S, LocalNeuron& L, ul
 		if(lane == 0) {
 			atomicAdd(&C.fired, (uint32_t) __popc(fb));
 			atomicAdd(&C.events, ev);
+			if(load) atomicAdd(&load[threadIdx.x >> 5], ev);
 		}
 	}
 	const uint32_t tb = __ballot_sync(0xffffffffu, target);
@@ -1602,9 +1607,16 @@ __device__ __forceinline__ bool local_update(const DevSim& S, LocalNeuron& L, ul
 		if(lane == 0) {
 			atomicOr(&S.touchedBits[L.n >> 5], tb);
 			atomicAdd(&C.stdp, se);
+			if(load) atomicAdd(&load[threadIdx.x >> 5], se);
 		}
 	}
 	return target;
+}
+
+// adds this warp's entries to those of its word of neurons
+__device__ __forceinline__ void keep_load(const DevSim& S, const LocalNeuron& L, const uint32_t* load)
+{
+	if((threadIdx.x & 31) == 0 && L.kind >= 0) atomicAdd(&S.warpLoad[L.n >> 5], load[threadIdx.x >> 5]);
 }
 
 // `steps` steps from cycle0, as run_kernel; the last step's deliveries stay
@@ -1615,11 +1627,12 @@ local_run_kernel(const DevSim S, const LocalLoop A)
 {
 	extern __shared__ __align__(16) unsigned char raw[];
 	__shared__ LocalCounters sC[2];  // by step parity: one is emptied while the other fills
-	__shared__ uint32_t sTarget, sOk;
+	__shared__ uint32_t sTarget, sOk, sLoad[32];
 	__shared__ unsigned long long sBar[2];
 	LocalNeuron L;
 	local_begin<SYNC>(S, A, raw, L);
 	if(threadIdx.x < 2) sC[threadIdx.x] = LocalCounters{ 0, 0, 0 };
+	if(threadIdx.x < 32) sLoad[threadIdx.x] = 0;
 	LoopBarrier<SYNC> bar(A.gb, &sTarget, &sOk, sBar, S.waitLimit, A.base);
 	const bool worker = threadIdx.x < A.workers, last = threadIdx.x >= blockDim.x - 32;
 	bool target = false;
@@ -1642,13 +1655,14 @@ local_run_kernel(const DevSim S, const LocalLoop A)
 		}
 		if(worker) {
 			target = local_update<SYNC, false>(S, L, S.slot2 + (size_t) cur * S.N, S.hist3 + (size_t) (c % 3) * S.N, c,
-					(uint32_t) (c % S.R), sC[cur]);
+					(uint32_t) (c % S.R), sC[cur], sLoad);
 		}
 	}
 	const unsigned long long end = A.cycle0 + A.steps;
 	if(worker) {
 		if(S.stdp) local_stdp(S, L, target, S.hist3 + (size_t) ((end + 1) % 3) * S.N);
 		local_end(S, L, (uint32_t) ((end - 1) & 1), false);
+		keep_load(S, L, sLoad);
 	}
 	__syncthreads();
 	if(threadIdx.x == 0) flush_counters(S, (uint32_t) ((end - 1) % S.R), sC[(end - 1) & 1]);
@@ -1665,11 +1679,12 @@ local_serve_kernel(const DevSim S, const LocalLoop A, ServeCtl* ctl, uint32_t se
 {
 	extern __shared__ __align__(16) unsigned char raw[];
 	__shared__ LocalCounters sC;
-	__shared__ uint32_t sTarget, sOk;
+	__shared__ uint32_t sTarget, sOk, sLoad[32];
 	__shared__ unsigned long long sBar[2];
 	LocalNeuron L;
 	local_begin<SYNC>(S, A, raw, L);
 	if(threadIdx.x == 0) sC = LocalCounters{ 0, 0, 0 };
+	if(threadIdx.x < 32) sLoad[threadIdx.x] = 0;
 	LoopBarrier<SYNC> bar(A.gb, &sTarget, &sOk, sBar, S.waitLimit, 0);
 	const bool worker = threadIdx.x < A.workers, last = threadIdx.x >= blockDim.x - 32;
 	uint32_t want = seq0;
@@ -1688,7 +1703,14 @@ local_serve_kernel(const DevSim S, const LocalLoop A, ServeCtl* ctl, uint32_t se
 		if(last) bar.arrive_and_wait([] {});
 		if(!bar.join()) break;
 		if(worker) {
-			target = local_update<SYNC, true>(S, L, S.slot2 + (size_t) cur * S.N, S.hist3 + (size_t) (c % 3) * S.N, c, ring, sC);
+			target = local_update<SYNC, true>(S, L, S.slot2 + (size_t) cur * S.N, S.hist3 + (size_t) (c % 3) * S.N, c, ring, sC,
+					sLoad);
+			// the host learns the busiest warp's entries
+			if(window_ends(c) && (threadIdx.x & 31) == 0 && L.kind >= 0) {
+				atomicMax(&A.gb->load, S.warpLoad[L.n >> 5] + sLoad[threadIdx.x >> 5]);
+				S.warpLoad[L.n >> 5] = 0;
+				sLoad[threadIdx.x >> 5] = 0;
+			}
 		}
 		__syncthreads();
 		if(last) {
@@ -1699,10 +1721,17 @@ local_serve_kernel(const DevSim S, const LocalLoop A, ServeCtl* ctl, uint32_t se
 		if(!bar.join()) break;
 		if(blockIdx.x == 0) {
 			answer_request(S, ctl, ring, hostIds, want);
+			if(window_ends(c) && threadIdx.x == 0) {
+				st_relaxed_sys_u64(&ctl->load, (unsigned long long) want << 32 | *(volatile uint32_t*) &A.gb->load);
+				A.gb->load = 0;
+			}
 		}
 	}
 	__syncthreads();
-	if(worker) local_end(S, L, (uint32_t) ((c - 1) & 1), true);
+	if(worker) {
+		local_end(S, L, (uint32_t) ((c - 1) & 1), true);
+		keep_load(S, L, sLoad);
+	}
 	bar.finish();
 }
 
@@ -1785,7 +1814,7 @@ __device__ __forceinline__ bool balanced_step(const DevSim& S, const LocalLoop& 
 	if(last) bar.arrive_and_wait([] {});
 	if(!bar.join()) return false;
 	if(worker) {
-		const bool target = local_update<2, STIM>(S, L, S.slot, S.hist + (size_t) cur * S.N, c, (uint32_t) (c % S.R), C);
+		const bool target = local_update<2, STIM>(S, L, S.slot, S.hist + (size_t) cur * S.N, c, (uint32_t) (c % S.R), C, nullptr);
 		balanced_publish(S, L, cur, target, reserve);
 	} else if(!last && more) {
 		local_noise(S, raw, A.workers, cur ^ 1u);
@@ -2216,6 +2245,8 @@ struct Collect {
 	unsigned long long* events;     // [chunk] (host)
 	unsigned long long* stdp;       // [chunk] (host)
 	const GridBarrier* barrier;     // null: none
+	uint32_t* load;                 // (host) the largest DevSim::warpLoad (null: not wanted)
+	uint32_t loadEnds;              // set them back to 0
 	uint32_t* error;                // (host) the barrier's error word
 };
 
@@ -2225,6 +2256,22 @@ collect_kernel(const DevSim S, const Collect C)
 	__shared__ uint32_t sIds[COLLECT_STAGE];
 	__shared__ uint32_t sWarp[COLLECT_THREADS / 32 + 1];
 	const uint32_t t = threadIdx.x, lane = t & 31, warp = t >> 5;
+	if(C.load && blockIdx.x == gridDim.x - 1) {
+		// a CTA of its own: the busiest warp of the single-barrier form
+		uint32_t most = 0;
+		for(uint32_t w = t; w < S.W; w += COLLECT_THREADS) {
+			most = max(most, S.warpLoad[w]);
+			if(C.loadEnds) S.warpLoad[w] = 0;
+		}
+		most = __reduce_max_sync(0xffffffffu, most);
+		if(lane == 0) sWarp[warp] = most;
+		__syncthreads();
+		if(t == 0) {
+			for(uint32_t w = 1; w < COLLECT_THREADS / 32; ++w) most = max(most, sWarp[w]);
+			*C.load = most;
+		}
+		return;
+	}
 	const uint32_t step = C.begin + blockIdx.x;
 	const uint32_t row = (C.ring0 + step) % S.R;
 	const uint32_t fired = S.firedCount[row];
@@ -3061,6 +3108,7 @@ void Simulation::init(const std::vector<const Network*>& nets, const Configurati
 	S.firedRing = dalloc<uint32_t>((size_t) S.R * S.W);
 	// the per-step counters, adjacent: one memset empties them
 	S.eventCount = dalloc<unsigned long long>((size_t) S.R * 3);
+	S.warpLoad = dalloc<uint32_t>(S.W);
 	S.stdpCount = S.eventCount + S.R;
 	S.firedCount = reinterpret_cast<uint32_t*>(S.stdpCount + S.R);
 	NB_CUDA(cudaMallocHost(&m_hFired, (size_t) S.W * 4));
@@ -3437,6 +3485,46 @@ void Simulation::launchLocal(unsigned n)
 	m_timerSteps += n;
 	m_stdpPending = false;
 	m_barrierUsed = true;
+	m_loadCounted |= !balanced;
+}
+
+// The single-barrier form is bound by its busiest warp: 2.1 us per round of 128
+// synapses or STDP entries.  Degrees bound that only at moderate rates.
+// run_kernel and serve_kernel deal the entries to all warps: 9 us a step, 12 us
+// per million events.  Microseconds a step, single barrier / run_kernel, half of
+// the neurons Poisson sources that fire with the given probability each ms:
+//   1000 x 100 0.06 6.8 / 9.2, 0.1 9.8 / 9.8, 0.3 21.7 / 12.4, 1 58.0 / 17.4;  2000 x
+//   400 0.1 28.8 / 10.3;  8000 x 300 0.1 21.2 / 11.7;  30000 x 100 0.1 11.2 / 12.1, 0.3
+//   23.1 / 18.1;  100k x 100 0.1 14.1 / 16.8, 0.3 28.0 / 28.3;  with STDP 1000 x 100 0.06
+//   10.9 / 11.3, 0.1 16.0 / 11.9, 100k x 100 0.03 14.8 / 16.2, 0.1 28.4 / 24.6
+// The two are even at 2.4 to 3.6 rounds a step of the busiest warp, at 8 with 1.6M
+// events (the example networks have 0.1 to 0.95).
+// So the simulation's own last BUSY_WINDOW steps or more decide: the busiest
+// warp's rounds turn to the other loops, fewer events by a margin turn back.
+constexpr double BUSY_ROUNDS = 2.7, BUSY_ROUNDS_PER_EVENT = 3e-6, BUSY_MARGIN = 0.6;
+
+// rounds: of the busiest warp in a step, on average over the window
+void Simulation::noteLoad(double rounds)
+{
+	const double events = (double) m_loadEvents / m_loadSteps;
+	if(m_busy ? events < BUSY_MARGIN * m_busyEvents : rounds > BUSY_ROUNDS + BUSY_ROUNDS_PER_EVENT * events) {
+		stopServe();
+		m_busy = !m_busy;
+		m_busyEvents = events;
+		m_knownSteps = 0;
+	} else {
+		m_knownSteps += m_loadSteps;
+	}
+	m_loadSteps = m_loadEvents = 0;
+}
+
+// Steps of run() until the next look at the load: soon while little is known.
+unsigned Simulation::stepsToLook() const
+{
+	if(!localRuns() || m_localSync == LOCAL_BALANCED) return ~0u;
+	// a warp of 32 neurons has at most 32 of their out- and in-degrees to do
+	if((m_maxOutDeg + (m_dev.stdp ? m_maxPlasticInDeg : 0)) / 4.0 < BUSY_ROUNDS) return ~0u;
+	return m_knownSteps < 2 * BUSY_WINDOW ? 2 * BUSY_WINDOW : m_knownSteps < 16 * BUSY_WINDOW ? 16 * BUSY_WINDOW : ~0u;
 }
 
 // After launches of the single-barrier loop: what the other loops' next step
@@ -3761,6 +3849,7 @@ void Simulation::launchServe()
 	// steps a launch the balanced form is ahead (187 / 192).
 	const bool local = localActive() && !(m_localSync == LOCAL_BALANCED && m_served == 1);
 	m_served = 0;
+	m_servingLists = !local || m_localSync == LOCAL_BALANCED;
 	if(local && m_localSync != LOCAL_BALANCED) flushStdp();  // of a step of another loop
 	else ensureLists();
 	NB_CUDA(cudaMemsetAsync(&m_barrier->count, 0, 8, m_stream));
@@ -3853,8 +3942,8 @@ void Simulation::stepResident(uint32_t nf, uint32_t ni)
 #endif
 		}
 	};
-	const uint32_t fired = tagged(c->reply[0]);
-	stepEvents += tagged(c->reply[1]);
+	const uint32_t fired = tagged(c->reply[0]), events = tagged(c->reply[1]);
+	stepEvents += events;
 	if(fired <= SERVE_TAGGED) {
 		m_fired.resize(fired);
 		for(uint32_t i = 0; i < fired; ++i) m_fired[i] = tagged(c->ids[i]);
@@ -3864,10 +3953,25 @@ void Simulation::stepResident(uint32_t nf, uint32_t ni)
 	}
 	m_serveSeq = serve_next(m_serveSeq);
 	++m_served;
+	// the single-barrier loop accumulates before it ends
+	m_stdpPending = m_servingLists;
 	m_cycle++;
 	m_timerSteps++;
-	// the single-barrier loop accumulates before it ends
-	m_stdpPending = !localActive() || m_localSync == LOCAL_BALANCED;
+	if(!m_servingLists || m_busy) {
+		++m_loadSteps;
+		m_loadEvents += events;
+		// a window's load arrives with its last answer or one of the next
+		const unsigned long long load = c->load;
+		const bool told = (uint32_t) (load >> 32) != m_loadTag;
+		m_loadTag = (uint32_t) (load >> 32);
+		if(m_busy) {
+			if(m_loadSteps >= BUSY_WINDOW) noteLoad(0);
+		} else if(told && m_loadSteps >= BUSY_WINDOW / 2) {
+			noteLoad((double) (uint32_t) load / 128 / m_loadSteps);
+		} else if(told) {
+			m_loadSteps = m_loadEvents = 0;  // too few for an average
+		}
+	}
 }
 
 // One step with host buffers: the stimulus is staged in mapped host memory
@@ -4023,7 +4127,8 @@ void Simulation::run(unsigned steps, unsigned stdpPeriod, float reward, unsigned
 	} inRun(m_inRun);
 	while(done < steps) {
 		const uint64_t first = m_cycle;
-		const unsigned chunk = std::min<unsigned>(steps - done, m_dev.R);
+		const unsigned chunk = std::min({ steps - done, (unsigned) m_dev.R, stepsToLook() });
+		m_loadCounted = false;
 		// the ring positions this chunk uses start at first % R and may wrap
 		NB_CUDA(cudaMemsetAsync(m_dev.eventCount, 0, (size_t) m_dev.R * 20, m_stream));
 		m_evUse.clear();
@@ -4062,12 +4167,19 @@ void Simulation::run(unsigned steps, unsigned stdpPeriod, float reward, unsigned
 		const uint32_t* hc = stepCounts();
 		const uint64_t* he = stepEventCounts();
 		const uint64_t* hs = he + m_dev.R;
+		uint64_t chunkEvents = 0;
 		for(unsigned i = 0; i < chunk; ++i) {
 			if(events) events[done + i] = he[i];
 			if(m_nets == 1 && counts) counts[done + i] = hc[i];
 			lastFired += hc[i];
 			lastEvents += he[i];
 			lastStdpEntries += hs[i];
+			chunkEvents += he[i];
+		}
+		if(m_loadCounted || m_busy) {
+			m_loadSteps += chunk;
+			m_loadEvents += chunkEvents;
+			if(m_loadSteps >= BUSY_WINDOW) noteLoad(m_loadCounted ? (double) *stepLoad() / 128 / m_loadSteps : 0);
 		}
 		// the ids of as many steps as the staging memory holds at a time
 		for(unsigned i = 0; i < chunk;) {
@@ -4108,9 +4220,11 @@ void Simulation::collect(uint64_t first, unsigned chunk, unsigned begin, bool id
 	c.events = reinterpret_cast<unsigned long long*>(m_dSteps);
 	c.stdp = c.events + m_dev.R;
 	c.counts = reinterpret_cast<uint32_t*>(c.stdp + m_dev.R);
-	c.error = c.counts + m_dev.R;
+	if(begin == 0 && m_loadCounted) c.load = c.counts + m_dev.R;
+	c.loadEnds = m_loadSteps + chunk >= BUSY_WINDOW;
+	c.error = c.counts + m_dev.R + 1;
 	c.barrier = m_barrier;
-	collect_kernel<<<chunk - begin, COLLECT_THREADS, 0, m_stream>>>(m_dev, c);
+	collect_kernel<<<chunk - begin + (c.load ? 1 : 0), COLLECT_THREADS, 0, m_stream>>>(m_dev, c);
 	NB_CUDA(cudaGetLastError());
 }
 
@@ -4141,6 +4255,7 @@ float Simulation::autotune(unsigned trialSteps)
 	}
 	if(m_dev.stdp) regions.emplace_back(m_dev.rcmAcc, (size_t) lastPlastic * 4);
 	regions.emplace_back(m_dev.touchedBits, (size_t) m_dev.W * 4);
+	regions.emplace_back(m_dev.warpLoad, (size_t) m_dev.W * 4);
 	std::vector<void*> backup;
 	for(auto& r : regions) {
 		void* p = nullptr;
@@ -4259,6 +4374,7 @@ float Simulation::autotune(unsigned trialSteps)
 	profiling = prof;
 	shapeLoop(bestP, bestT);
 	m_localOn = pers && m_localRuns ? bestLocal : local0;
+	m_busy = false;  // the trials saw the load
 	m_fusedOn = pers ? fused0 : bestLocal;
 	return best * 1e3f / trialSteps;
 }

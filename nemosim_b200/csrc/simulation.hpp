@@ -30,7 +30,8 @@ struct GridBarrier {
 	uint32_t cmd;    // resident step loop: the request being run (| stop flag: end)
 	uint32_t error;  // set when a wait gave up
 	uint32_t nf, ni; // resident step loop: the request's stimulus sizes
-	uint32_t pad[3];
+	uint32_t load;   // resident step loop, single-barrier form: the busiest warp's entries of a window
+	uint32_t pad[2];
 };
 static_assert(offsetof(GridBarrier, cmd) == 4, "one memset restarts count and cmd");
 
@@ -55,6 +56,9 @@ constexpr unsigned RESIDENT_REPLY_LIMIT_S = 20;
 // poll that finds the request also reads it: inl[i] = seq << 32 | local
 // index, each word checked by its sequence number as the request words
 // are, and req[0]'s low half is then SERVE_INLINE_FLAG | count.
+// steps after which the load of the single-barrier form is looked at
+constexpr uint32_t BUSY_WINDOW = 32;
+__host__ __device__ inline bool window_ends(unsigned long long cycle) { return cycle % BUSY_WINDOW == BUSY_WINDOW - 1; }
 constexpr uint32_t SERVE_TAGGED = 4096;  // fired ids that an answer carries word by word
 constexpr uint32_t SERVE_INLINE = 6;
 constexpr uint32_t SERVE_INLINE_FLAG = 0x80000000u;
@@ -65,7 +69,10 @@ struct ServeCtl {
 	// the answer: sequence number << 32 | fired neurons, then | synaptic
 	// events, then (up to SERVE_TAGGED of them) | each fired global id
 	unsigned long long reply[2];
-	unsigned long long pad1[14];
+	// after a window of the single-barrier form: sequence number << 32 | the
+	// busiest warp's entries
+	unsigned long long load;
+	unsigned long long pad1[13];
 	unsigned long long ids[SERVE_TAGGED];
 };
 static_assert(offsetof(ServeCtl, inl) + 8 * SERVE_INLINE <= 64, "the request and its inline stimulus share one 64-byte line");
@@ -140,6 +147,7 @@ struct DevSim {
 	uint32_t* firedIds;       // [N] staging of a step's fired global ids
 	uint32_t l2gIdentity;     // l2g[i] == i for every neuron
 	uint32_t* firedCount;     // [R]
+	uint32_t* warpLoad;             // [W] entries of each word's warp in the window, single-barrier form (noteLoad)
 	unsigned long long* eventCount; // [R] synaptic events (out-degree of fired neurons)
 	unsigned long long* stdpCount;  // [R] incoming plastic synapses walked by STDP
 	int stdp;
@@ -263,7 +271,7 @@ public:
 	const char* stepKernel() const;
 	bool persistentActive() const { return usePersistent && m_runGrid != 0; }
 	// the persistent loop's steps run through its single-barrier form
-	bool localActive() const { return persistentActive() && m_localOn; }
+	bool localActive() const { return persistentActive() && m_localOn && !m_busy; }
 	// those of run(), not only those of nemo_step
 	bool localRuns() const { return localActive() && m_localRuns; }
 	// step() keeps the persistent loop resident on the GPU between calls
@@ -369,6 +377,16 @@ private:
 	int m_localSync = 2;
 	uint32_t m_localWorkers = 0, m_localT = 0, m_localGrid = 0, m_localStride = 0;
 	size_t m_localSmem = 0;
+	// whether the single-barrier form stands back (noteLoad), and the events per
+	// step when it did; steps and events of the window, steps since the last
+	// change; whether the chunk has steps of that form
+	bool m_busy = false, m_loadCounted = false;
+	double m_busyEvents = 0;
+	uint64_t m_loadSteps = 0, m_loadEvents = 0, m_knownSteps = 0;
+	uint32_t m_loadTag = 0;  // sequence number of the last load that the resident loop told
+	void noteLoad(double rounds);
+	unsigned stepsToLook() const;
+	bool m_servingLists = false;  // the resident loop in use leaves work lists and STDP entries behind
 	uint64_t m_served = 0;      // steps of the resident loop's last launch
 	bool m_listsStale = false;  // its launches left the other loops' work lists behind
 	// STDP over a delay of 64 (which an empty post-fire part allows) reads the
@@ -399,11 +417,12 @@ private:
 	uint32_t* m_hStage = nullptr;    // mapped pinned: results on their way to the caller
 	uint32_t* m_dStage = nullptr;
 	size_t m_stageCap = 0;           // words
-	uint64_t* m_hSteps = nullptr;    // mapped pinned: events [R], STDP entries [R], fired counts [R] u32, error word
+	uint64_t* m_hSteps = nullptr;    // mapped pinned: events [R], STDP entries [R], fired counts [R] u32, load, error word
 	uint64_t* m_dSteps = nullptr;
 	const uint64_t* stepEventCounts() const { return m_hSteps; }
 	const uint32_t* stepCounts() const { return reinterpret_cast<const uint32_t*>(m_hSteps + 2 * (size_t) m_dev.R); }
-	const uint32_t* stepError() const { return stepCounts() + m_dev.R; }
+	const uint32_t* stepLoad() const { return stepCounts() + m_dev.R; }
+	const uint32_t* stepError() const { return stepLoad() + 1; }
 	uint32_t* m_streamOrder = nullptr;
 	uint32_t* m_streamNet = nullptr;
 	uint32_t* m_netCounts = nullptr; // [R][nets]

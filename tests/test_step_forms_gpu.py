@@ -44,14 +44,15 @@ def test_form_and_results(n, fanout, dmax, stdp, form, one_kernel):
     sp, so = nb.Simulation(pn, conf(nb, stdp)), O.Simulation(on, conf(O, stdp))
     assert sp.step_kernel() == form
     assert_same(sp, so, parts, 60, 25 if stdp else 0, n)
-    assert sp.step_kernel() == form
+    after = sp.step_kernel()
+    assert after in (form, "run_kernel")  # the latter where those steps were busy
     sp.set_persistent(False)
     assert sp.step_kernel() == ("fused_step_kernel" if one_kernel else "update_kernel")
     assert_same(sp, so, parts, 30, 25 if stdp else 0, n)
     sp.set_launch(64, 96)
     assert sp.step_kernel() == "update_kernel"
     sp.set_persistent(True)
-    assert sp.step_kernel() == form
+    assert sp.step_kernel() == after
     sp.set_launch(64, 96)
     assert sp.step_kernel() == "run_kernel"
     assert_same(sp, so, parts, 30, 25 if stdp else 0, n)
