@@ -3195,7 +3195,10 @@ void Simulation::init(const std::vector<const Network*>& nets, const Configurati
 			usePersistent = false;
 			// one neuron per thread in many small CTAs, against two
 			// partitions per SM: 23.0 / 29.8 us a step at 400k neurons
+			m_wideP = m_P;
+			m_wideT = m_T;
 			shapeLoop(128, 128);
+			m_ownShape = true;
 		}
 		if(m_runGrid) planLocal();
 	}
@@ -3521,6 +3524,7 @@ void Simulation::noteLoad(double rounds)
 // Steps of run() until the next look at the load: soon while little is known.
 unsigned Simulation::stepsToLook() const
 {
+	if(m_ownShape && m_dev.stdp && !m_fusedOn && !m_shapeKnown && !persistentActive()) return GRAPH_STEPS;
 	if(!localRuns() || m_localSync == LOCAL_BALANCED) return ~0u;
 	// a warp of 32 neurons has at most 32 of their out- and in-degrees to do
 	if((m_maxOutDeg + (m_dev.stdp ? m_maxPlasticInDeg : 0)) / 4.0 < BUSY_ROUNDS) return ~0u;
@@ -3555,8 +3559,28 @@ void Simulation::setLaunch(uint32_t P, uint32_t T)
 	if(P != partition() || T != threads()) shapeLoop(P, T);
 }
 
+// The two-launch step of a large network without a shape of the caller's: 128
+// neurons per CTA, or two partitions per SM while it learns and fires often (in
+// the lists of many small partitions neighbours are further apart).
+// Microseconds a step, 128 / two per SM, with STDP: example networks (0.5% to
+// 0.7% of the neurons a step) 160k x 300 20.5 / 24.6, 300k x 300 34.8 / 35.7, 400k x
+// 500 47.0 / 55.3; 300k x 200 with 1.4% 40.3 / 38.4, 6% 97 / 83; 200k x 300 with 3.4%
+// 61 / 51, 6% 90 / 71.  Without STDP 300k x 500 with 6% 86.7 / 90.7.
+constexpr double OWN_SHAPE_BUSY = 0.012, OWN_SHAPE_CALM = 0.009;
+
+void Simulation::noteFired(double share)
+{
+	if(!m_ownShape || !m_dev.stdp || persistentActive() || m_fusedOn) return;
+	m_shapeKnown = true;
+	const bool wide = m_P != 128;
+	if(wide ? share >= OWN_SHAPE_CALM : share <= OWN_SHAPE_BUSY) return;
+	shapeLoop(wide ? 128 : m_wideP, wide ? 128 : m_wideT);
+	m_ownShape = true;
+}
+
 void Simulation::shapeLoop(uint32_t P, uint32_t T)
 {
+	m_ownShape = false;
 	stopServe();
 	if(persistentActive()) {
 		m_localOn = false;  // the caller shapes the persistent loop
@@ -4167,7 +4191,7 @@ void Simulation::run(unsigned steps, unsigned stdpPeriod, float reward, unsigned
 		const uint32_t* hc = stepCounts();
 		const uint64_t* he = stepEventCounts();
 		const uint64_t* hs = he + m_dev.R;
-		uint64_t chunkEvents = 0;
+		uint64_t chunkEvents = 0, chunkFired = 0;
 		for(unsigned i = 0; i < chunk; ++i) {
 			if(events) events[done + i] = he[i];
 			if(m_nets == 1 && counts) counts[done + i] = hc[i];
@@ -4175,7 +4199,9 @@ void Simulation::run(unsigned steps, unsigned stdpPeriod, float reward, unsigned
 			lastEvents += he[i];
 			lastStdpEntries += hs[i];
 			chunkEvents += he[i];
+			chunkFired += hc[i];
 		}
+		noteFired((double) chunkFired / chunk / m_N);
 		if(m_loadCounted || m_busy) {
 			m_loadSteps += chunk;
 			m_loadEvents += chunkEvents;

@@ -434,6 +434,11 @@ private:
 	unsigned m_deliverGrid = 1184;  // CTAs of deliver_kernel
 	unsigned m_applyGrid = 1184;    // CTAs of apply_kernel
 	uint32_t m_P = 256, m_T = 256;
+	// whether the shape of the two-launch step is noteFired's to choose; two
+	// partitions per SM; whether it has seen the network's rates
+	bool m_ownShape = false, m_shapeKnown = false;
+	uint32_t m_wideP = 0, m_wideT = 0;
+	void noteFired(double share);
 	uint32_t m_maxOutDeg = 0, m_maxPlasticInDeg = 0;
 	uint32_t m_noisyWords = 0;  // words of 32 neurons with an Izhikevich neuron that has input noise at construction
 	int m_sms = 148;

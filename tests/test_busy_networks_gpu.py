@@ -97,3 +97,44 @@ def test_nemo_step(n, form, stdp):
     assert a.step_kernel() == "run_kernel"
     assert a.step_events() == b.step_events()
     same_end(a, b, n, fanout, stdp)
+
+
+def test_two_launch_shape_of_a_large_learning_network():
+    """Without a shape of the caller's, the two-launch step of a large network
+    with STDP takes wider partitions while the network fires often."""
+    n, sources = 230_000, 11_500
+    rng = np.random.default_rng(3)
+
+    def build():
+        net = nb.Network()
+        ids = np.arange(n, dtype=np.uint32)
+        net.add_neuron(net.add_neuron_type("PoissonSource"), ids[:sources], np.float32(0.6))
+        net.add_neuron(net.add_neuron_type("IzhikevichRS"), ids[sources:], -13.0, -65.0)
+        r = np.random.default_rng(4)
+        # a hub of out-degree 401: not one kernel per step
+        src = np.concatenate([np.repeat(ids, 3), np.full(398, 9)]).astype(np.uint32)
+        net.add_synapse(src, r.integers(0, n, len(src)).astype(np.uint32), r.integers(1, 21, len(src)).astype(np.uint32),
+                        np.full(len(src), 2.0, np.float32), np.ones(len(src), np.uint8))
+        return nb.Simulation(net, nets.standard_stdp(nb))
+
+    a, b = build(), build()
+    b.set_persistent(False)
+    b.set_launch(256, 256)
+    assert a.step_kernel() == "update_kernel" and a.launch() == (128, 128)
+    a.set_launch(*a.launch())  # changes nothing
+    same(a, b, 130, 50, n)
+    wide = a.launch()
+    assert wide[0] > 256 and wide[1] > 256
+    same(a, b, 130, 50, n)
+    assert a.launch() == wide
+    for s in (a, b):
+        for i in rng.permutation(sources).tolist():
+            s.set_neuron_parameter(i, 0, 0.001)
+    same(a, b, 130, 50, n)
+    assert a.launch() == (128, 128)
+    same(a, b, 30, 0, n)
+    assert list(a.step([5])) == list(b.step([5]))
+    a.set_launch(96, 96)
+    same(a, b, 20, 0, n)
+    assert a.launch() == (96, 96)
+    assert np.array_equal(a.weights_fx(3 * n + 398), b.weights_fx(3 * n + 398))
