@@ -195,22 +195,36 @@ __device__ __forceinline__ unsigned load_mask(const BpttDev& D, const unsigned c
 
 // the general form: counts from the spike words, every synapse added -- for
 // neurons that fired more than once in some ms of the window, and for
-// weights that are not finite (inf x 0 is NaN)
+// weights that are not finite (inf x 0 is NaN).  Each lane loads the word and
+// the weight of one synapse, 32 at a time; the lanes of the trials then take
+// them by shuffles, in order.  (A word at a time, every lane loading the same,
+// was bound by one L2 round trip per synapse: a gradient of 30000 x 20, 100 ms,
+// one trial 6.6 ms against 3.7, of 2000 x 100, 200 ms, 16 trials 10.6 against 4.3)
 template<typename Real, typename Entry, typename Weight>
 __device__ __noinline__ Real gather_counts(const BpttDev& D, const unsigned char* words, int g, const Entry* list,
 		const Weight* w, int len, int t)
 {
 	const int lane = threadIdx.x & 31, b = lane & (D.lanes - 1), main = len & ~3;
+	const unsigned FULL = 0xffffffffu;
 	Real s[4] = { Real(0), Real(0), Real(0), Real(0) };
-	for(int k = 0; k < len; ++k) {
-		const int2 e = unpack_synapse(list[k]);
-		Real x = Real(0);
-		if(t >= e.y) {
-			x = (Real) ((int) (load_word(words, ((size_t) (t - e.y) * D.groups + g) * D.N + e.x, D.wordLog) >> (4 * b)) & 15);
+	for(int k0 = 0; k0 < len; k0 += 32) {
+		unsigned long long word = 0;
+		Real wk = Real(0);
+		if(k0 + lane < len) {
+			const int2 e = unpack_synapse(list[k0 + lane]);
+			wk = (Real) w[k0 + lane];
+			if(t >= e.y) word = load_word(words, ((size_t) (t - e.y) * D.groups + g) * D.N + e.x, D.wordLog);
 		}
-		const int j = k < main ? k & 3 : 0;
+		auto term = [&](int i, Real sum) {
+			const Real x = (Real) ((int) (__shfl_sync(FULL, word, i) >> (4 * b)) & 15);
+			return fma(__shfl_sync(FULL, wk, i), x, sum);
+		};
+		const int n = min(32, len - k0), quads = min(n, main - k0);
+		for(int i = 0; i < quads; i += 4) {
 #pragma unroll
-		for(int q = 0; q < 4; ++q) if(j == q) s[q] = fma((Real) w[k], x, s[q]);
+			for(int q = 0; q < 4; ++q) s[q] = term(i + q, s[q]);
+		}
+		for(int i = max(quads, 0); i < n; ++i) s[0] = term(i, s[0]);
 	}
 	return (s[0] + s[2]) + (s[1] + s[3]);
 }
