@@ -9,10 +9,10 @@ pytestmark = pytest.mark.gpu
 
 
 # in-degrees around 32 and 64 and of 100 and 2500, one to 20 trials, more
-# neurons than a CTA's warps hold
+# neurons than a CTA's warps hold, and (the last two) than half of its threads
 @pytest.mark.parametrize("neurons,fanout,ms,trials,readout", [
     (70, 31, 20, 4, 10), (70, 33, 20, 1, 10), (90, 64, 20, 20, 10), (500, 100, 15, 7, 40), (40, 2500, 12, 4, 8),
-    (6000, 20, 12, 1, 60)])
+    (6000, 20, 12, 1, 60), (76_000, 5, 10, 1, 60), (4800, 13, 12, 16, 60)])
 def test_counts_match_autograd(neurons, fanout, ms, trials, readout):
     dev, net, model, noise, target = setup(neurons=neurons, fanout=fanout, ms=ms, trials=trials, readout=readout,
                                            smooth=False, ckpt=7, state_dtype=torch.float64)
