@@ -196,17 +196,20 @@ __device__ __forceinline__ unsigned load_mask(const BpttDev& D, const unsigned c
 // the general form: counts from the spike words, every synapse added -- for
 // neurons that fired more than once in some ms of the window, and for
 // weights that are not finite (inf x 0 is NaN).  Each lane loads the word and
-// the weight of one synapse, 32 at a time; the lanes of the trials then take
-// them by shuffles, in order.  (A word at a time, every lane loading the same,
-// was bound by one L2 round trip per synapse: a gradient of 30000 x 20, 100 ms,
-// one trial 6.6 ms against 3.7, of 2000 x 100, 200 ms, 16 trials 10.6 against 4.3)
+// the weight of one synapse, 32 at a time; the lanes (sub, trial) then take the
+// partial sums sub (and sub + 2) from them by shuffles, in order.  (A word at a
+// time, every lane loading the same, was bound by one L2 round trip per
+// synapse: a gradient of 30000 x 20, 100 ms, one trial 6.6 against 2.3 ms, of 2000 x 100,
+// 200 ms, 16 trials 10.6 against 3.9.  Out of line, and called per neuron: the usual path
+// beside it lost 1.5% to a second loop over the neurons.)
 template<typename Real, typename Entry, typename Weight>
 __device__ __noinline__ Real gather_counts(const BpttDev& D, const unsigned char* words, int g, const Entry* list,
 		const Weight* w, int len, int t)
 {
-	const int lane = threadIdx.x & 31, b = lane & (D.lanes - 1), main = len & ~3;
 	const unsigned FULL = 0xffffffffu;
-	Real s[4] = { Real(0), Real(0), Real(0), Real(0) };
+	const int lane = threadIdx.x & 31, b = lane & (D.lanes - 1), main = len & ~3;
+	const int sub = (lane >> (31 - __clz(D.lanes))) & 3, subs = D.lanes > 8 ? 2 : 4;
+	Real s0 = Real(0), s1 = Real(0);
 	for(int k0 = 0; k0 < len; k0 += 32) {
 		unsigned long long word = 0;
 		Real wk = Real(0);
@@ -219,46 +222,19 @@ __device__ __noinline__ Real gather_counts(const BpttDev& D, const unsigned char
 			const Real x = (Real) ((int) (__shfl_sync(FULL, word, i) >> (4 * b)) & 15);
 			return fma(__shfl_sync(FULL, wk, i), x, sum);
 		};
-		const int n = min(32, len - k0), quads = min(n, main - k0);
+		const int n = min(32, len - k0), quads = max(0, min(n, main - k0));
 		for(int i = 0; i < quads; i += 4) {
-#pragma unroll
-			for(int q = 0; q < 4; ++q) s[q] = term(i + q, s[q]);
+			s0 = term(i + sub, s0);
+			if(subs == 2) s1 = term(i + sub + 2, s1);
 		}
-		for(int i = max(quads, 0); i < n; ++i) s[0] = term(i, s[0]);
+		for(int i = quads; i < n; ++i) {
+			const Real x = term(i, s0);
+			if(sub == 0) s0 = x;
+		}
 	}
-	return (s[0] + s[2]) + (s[1] + s[3]);
-}
-
-// The same by one thread per (neuron, trial), eight words in flight: a warp per
-// neuron does the work of 32 lanes for the few trials.  For up to COUNT_LANES
-// trials, where the CTA has items for half of its threads.  Microseconds a ms of
-// the forward pass, thread / warp, a fifth of the neurons firing: 100k x 10, one
-// trial 16.7 / 39.1, 78k x 100, one trial 127 / 175, 100k x 20, 4 trials 47 / 53, 12k x
-// 50, 8 trials 19.1 / 19.4, 20k x 50, 16 trials 69 / 38.
-constexpr int COUNT_ITEMS = LOOP_THREADS / 2, COUNT_LANES = 4;
-
-template<typename Real, typename Entry, typename Weight>
-__device__ __noinline__ Real gather_counts_alone(const BpttDev& D, const unsigned char* words, int g, const Entry* list,
-		const Weight* w, int len, int t, int b)
-{
-	const int main = len & ~3;
-	Real s[4] = { Real(0), Real(0), Real(0), Real(0) };
-	auto load = [&](int k) -> unsigned long long {
-		const int2 e = unpack_synapse(list[k]);
-		return t >= e.y ? load_word(words, ((size_t) (t - e.y) * D.groups + g) * D.N + e.x, D.wordLog) : 0ull;
-	};
-	auto term = [&](int k, unsigned long long word, Real sum) {
-		return fma((Real) w[k], (Real) ((int) (word >> (4 * b)) & 15), sum);
-	};
-	for(int k0 = 0; k0 < main; k0 += 8) {
-		unsigned long long word[8];
-#pragma unroll
-		for(int q = 0; q < 8; ++q) word[q] = k0 + q < main ? load(k0 + q) : 0ull;
-#pragma unroll
-		for(int q = 0; q < 8; ++q) if(k0 + q < main) s[q & 3] = term(k0 + q, word[q], s[q & 3]);
-	}
-	for(int k = main; k < len; ++k) s[0] = term(k, load(k), s[0]);
-	return (s[0] + s[2]) + (s[1] + s[3]);
+	if(subs == 2) s0 += s1;
+	else s0 += __shfl_xor_sync(FULL, s0, 2 * D.lanes);
+	return s0 + __shfl_xor_sync(FULL, s0, D.lanes);
 }
 
 // masks: all slices (global memory); window, slot: the last D.ring of them by
@@ -670,12 +646,7 @@ bptt_forward_loop(const BpttDev D, const BpttState<Real> X, const BpttParams P, 
 				if(more) lastMulti = t - 1;
 			}
 			const bool counts = all || t - lastMulti <= D.ring;
-			const bool alone = counts && lanes <= COUNT_LANES && items >= COUNT_ITEMS;
-			for(int i = tid; alone && i < items; i += LOOP_THREADS) {
-				const int2 at = place(i >> laneLog);
-				in[i] = gather_counts_alone<Real>(D, X.words, g, list + at.x, weight + at.x, at.y, t, i & (lanes - 1));
-			}
-			if(!alone) for(int cl = warp; cl < nc; cl += LOOP_THREADS / 32) {
+			for(int cl = warp; cl < nc; cl += LOOP_THREADS / 32) {
 				const int2 at = place(cl);
 				const Real s = counts ? gather_counts<Real>(D, X.words, g, list + at.x, weight + at.x, at.y, t)
 						: gather_masks<Real, MODE>(D, X.masks, window, slot, g, list + at.x, weight + at.x, at.y, t, lists);
@@ -738,18 +709,18 @@ bptt_forward_loop(const BpttDev D, const BpttState<Real> X, const BpttParams P, 
 					for(int o = 1; o < lanes; o <<= 1) word |= __shfl_xor_sync(0xffffffffu, word, o);
 				}
 				const unsigned fired = __ballot_sync(0xffffffffu, count != 0);
-				const size_t slice = (size_t) t * D.groups + g;
-				// one plain store a warp (every one is a 1): an atomic by each
-				// neuron queued 100k of them at one address, 30 us a ms
-				if(__any_sync(0xffffffffu, count > 1) && lane == 0) {
-					*reinterpret_cast<volatile unsigned*>(X.masks + slice * D.maskStride) = 1u;
-				}
+				const bool more = __any_sync(0xffffffffu, count > 1);
 				if(act && bl == 0) {
+					const size_t slice = (size_t) t * D.groups + g;
 					store_word(X.words, slice * D.N + n, D.wordLog, word);
 					unsigned char* masks = X.masks + slice * D.maskStride;
 					const unsigned m = fired >> (lane & ~(lanes - 1)) & ((1u << lanes) - 1u);
 					if(lanes > 8) reinterpret_cast<uint16_t*>(masks + MASK_HEADER)[n] = (uint16_t) m;
 					else masks[MASK_HEADER + n] = (unsigned char) m;
+					// one plain store a warp (every one is a 1): an atomic by each
+					// neuron queued 100k of them at one address, 30 us a ms.  (A
+					// warp that has fired twice has an item in lane 0.)
+					if(more && lane == 0) *reinterpret_cast<volatile unsigned*>(masks) = 1u;
 				}
 			}
 		}

@@ -8,8 +8,8 @@ from tests.test_bptt_gpu import TOL, reference, relerr, setup
 pytestmark = pytest.mark.gpu
 
 
-# in-degrees around 32 and 64 and of 100 and 2500, one to 20 trials, more
-# neurons than a CTA's warps hold, and (the last two) than half of its threads
+# in-degrees around 32 and 64 and of 100 and 2500, one to 20 trials (every split of a list's four sums over lanes), more
+# neurons than a CTA's warps hold
 @pytest.mark.parametrize("neurons,fanout,ms,trials,readout", [
     (70, 31, 20, 4, 10), (70, 33, 20, 1, 10), (90, 64, 20, 20, 10), (500, 100, 15, 7, 40), (40, 2500, 12, 4, 8),
     (6000, 20, 12, 1, 60), (76_000, 5, 10, 1, 60), (4800, 13, 12, 16, 60)])
