@@ -25,8 +25,9 @@ wall second.
            launches per call)
   roofline the step loop's algorithmic bytes per launch / its measured
            average duration (CUDA events around each launch), against the
-           measured HBM copy bandwidth; the persistent loop runs one period
-           per launch
+           measured HBM copy bandwidth; a cooperative loop runs one period
+           per launch.  kernel: the one that runs (Simulation.step_kernel)
+  phases_us  one traced launch of run_kernel, where that is the timed kernel
   --impl reference  the CPU oracle (a restatement of the reference CPU
            backend; the reference itself cannot be built here) on the host
 
@@ -358,12 +359,22 @@ def run_b200(args, rank, world, local):
     ps = sim.run_stats()
     steps_p = kp * W
     persistent = ps["kernel_launches"]["run"] > 0
+    step_kernel = sim.step_kernel()
     if persistent:
-        # one launch of the persistent step loop per STDP period
+        # one launch of the step loop per STDP period; run_kernel reads and
+        # writes its neurons every step, the forms that keep them on chip once
+        # a launch
         nl = ps["kernel_launches"]["run"]
-        run_bytes = (args.neurons * B_NEURON * steps_p + ps["fired"] * B_FIRED + ps["events"] * B_EVENT
+        neuron_steps = steps_p if step_kernel == "run_kernel" else nl
+        run_bytes = (args.neurons * B_NEURON * neuron_steps + ps["fired"] * B_FIRED + ps["events"] * B_EVENT
                      + ps["stdp_entries"] * B_STDP) / nl
-        kernels = {"run_kernel": (run_bytes, ps["kernel_ms"]["run"] / nl)}
+        kernels = {step_kernel: (run_bytes, ps["kernel_ms"]["run"] / nl)}
+    elif step_kernel == "fused_step_kernel":
+        # one launch a step, and one per segment for the deliveries to its first
+        nl = max(1, ps["kernel_launches"]["step"])
+        run_bytes = (args.neurons * B_NEURON * nl + ps["fired"] * B_FIRED + ps["events"] * B_EVENT
+                     + ps["stdp_entries"] * B_STDP) / nl
+        kernels = {step_kernel: (run_bytes, ps["kernel_ms"]["step"] / nl)}
     else:
         nsteps_p = max(1, ps["kernel_launches"]["step"])
         upd_ms = ps["kernel_ms"]["step"] / nsteps_p
@@ -390,9 +401,9 @@ def run_b200(args, rank, world, local):
                       "achieved_gbs": v[0] / (v[1] / 1e3) / 1e9 if v[1] else None} for k, v in kernels.items()}
     per_kernel["apply_kernel"] = {"avg_launch_us": apply_ms * 1e3, "achieved_gbs": apply_gbs,
                                   "alg_bytes_per_launch": ps["plastic_synapses"] * B_APPLY}
-    # where a step's time goes: one traced launch of the persistent loop
+    # where a step's time goes: one traced launch of run_kernel
     phases = None
-    if persistent:
+    if step_kernel == "run_kernel":
         phases = phase_summary(sim.trace_phases(W))
 
     # e2e through the C ABI with host buffers, the calls a C program makes:
@@ -480,9 +491,11 @@ def run_b200(args, rank, world, local):
                     "step_path": "resident step loop" if resident else "two launches per nemo_step",
                     "sim_ms_per_s": ke * W / e2e_s, "fired_per_ms": fired_total / (ke * W),
                     "python_step_us": py_step_us},
-            # per period: the persistent loop (or 100 update + deliver launches,
-            # plus the graph's cycle-counter kernel), then applyStdp's kernel
-            "gpu_launches": args.steps * ((1 if persistent else 2 * W + (W // 100)) + 1),
+            # per period: the step loop (or 100 launches of one or two kernels
+            # plus the graph's cycle-counter kernel), then applyStdp's kernel;
+            # per 1024 steps the kernel that collects the results
+            "gpu_launches": args.steps * ((1 if persistent else len(kernels) * W + (W // 100)) + 1)
+            + -(-args.steps * W // 1024),
             "clocks": clk.summary(),
             # network generation (the random example's own loop, on the host)
             # and the simulation's construction from it, both untimed
@@ -492,8 +505,8 @@ def run_b200(args, rank, world, local):
             "phases_us": phases,
             "launch": {"partition": launch[0], "threads": launch[1],
                        "autotuned_us_per_step": tuned_us,
-                       "step_loop": "persistent cooperative launch per period" if persistent
-                       else "two launches per step" + ("" if args.no_graphs else ", CUDA graphs of 100 steps")},
+                       "step_loop": step_kernel + (", a cooperative launch per period" if persistent
+                                                   else "" if args.no_graphs else ", CUDA graphs of 100 steps")},
             "spikes_per_neuron_s": st["fired"] / args.neurons / (args.steps * W / 1e3),
         }
     del sim
@@ -573,14 +586,16 @@ def run_batch(args, local, emit=True):
     streams = batch.streams(counts, ids)
     mismatched = sum(1 for (c1, i1), (c2, i2) in zip(streams, seq)
                      if not (np.array_equal(c1, c2) and np.array_equal(i1, i2)))
-    # the same batch continued with each step loop in turn (the default
-    # above is the persistent loop unless the batch has more than two neurons
-    # per resident thread)
+    # the same batch continued with a cooperative loop and with launches per
+    # step (the default above is the former unless the batch has more than two
+    # neurons per resident thread)
+    step_kernel = batch.step_kernel()
     loop_ms = {}
     for persistent in (True, False):
         batch.set_persistent(persistent)
+        name = batch.step_kernel()
         batch.run(ms, ids=False)
-        loop_ms["persistent" if persistent else "two_launch_graphs"] = batch.run_stats()["run_ms"]
+        loop_ms[name] = batch.run_stats()["run_ms"]
     synapses = sum(sp["n"] * sp["f"] for sp in specs)
     # algorithmic bytes of the checked run (no STDP): neuron-steps, the
     # fired neurons' c and d, synaptic events
@@ -600,7 +615,7 @@ def run_batch(args, local, emit=True):
         "batch_events_per_s": st["events"] / (batch_ms / 1e3),
         "bitexact_vs_individual_runs": mismatched == 0, "mismatched_networks": mismatched,
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-                     "traffic": None, "peak_kind": peak_kind, "alg_bytes": alg},
+                     "traffic": None, "peak_kind": peak_kind, "alg_bytes": alg, "kernel": step_kernel},
         "launch": {"partition": launch[0], "threads": launch[1], "autotuned_us_per_step": tuned_us},
         "batch_build_s": build_s, "clocks": clk.summary(),
     }
