@@ -93,8 +93,8 @@ __host__ __device__ inline int sync_counter(int group, bool backward, int maxGro
 	return SYNC_STRIDE * (1 + group + (backward ? maxGroups : 0));
 }
 
-// Waits give up after this many polls (about a minute; a millisecond of the
-// loop takes microseconds)
+// Waits give up after this many polls (eleven seconds at 171 ns a poll; a
+// millisecond of the loop takes microseconds)
 constexpr unsigned LOOP_POLL_LIMIT = 1u << 26;
 
 // One launch of a loop: CTAs and neurons per trial group, the first group,
