@@ -693,6 +693,7 @@ nemo_status_t nemo_b200_get_launch(nemo_simulation_t s, unsigned* partition, uns
 nemo_status_t nemo_b200_get_step_kernel(nemo_simulation_t s, const char** name)
 {
 	NULLCHECK(s);
+	NULLCHECK(name);
 	CALL(*name = S(s).stepKernel());
 }
 
