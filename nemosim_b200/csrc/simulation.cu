@@ -1705,9 +1705,11 @@ local_serve_kernel(const DevSim S, const LocalLoop A, ServeCtl* ctl, uint32_t se
 		if(worker) {
 			target = local_update<SYNC, true>(S, L, S.slot2 + (size_t) cur * S.N, S.hist3 + (size_t) (c % 3) * S.N, c, ring, sC,
 					sLoad);
-			// the host learns the busiest warp's entries
+			// the host learns the busiest warp's entries, where they could
+			// matter (two rounds a step and more)
 			if(window_ends(c) && (threadIdx.x & 31) == 0 && L.kind >= 0) {
-				atomicMax(&A.gb->load, S.warpLoad[L.n >> 5] + sLoad[threadIdx.x >> 5]);
+				const uint32_t entries = S.warpLoad[L.n >> 5] + sLoad[threadIdx.x >> 5];
+				if(entries > 2 * 128 * BUSY_WINDOW) atomicMax(&A.gb->load, entries);
 				S.warpLoad[L.n >> 5] = 0;
 				sLoad[threadIdx.x >> 5] = 0;
 			}
@@ -3512,6 +3514,8 @@ void Simulation::noteLoad(double rounds)
 	const double events = (double) m_loadEvents / m_loadSteps;
 	if(m_busy ? events < BUSY_MARGIN * m_busyEvents : rounds > BUSY_ROUNDS + BUSY_ROUNDS_PER_EVENT * events) {
 		stopServe();
+		// what a resident loop has counted since its last window
+		NB_CUDA(cudaMemsetAsync(m_dev.warpLoad, 0, (size_t) m_dev.W * 4, m_stream));
 		m_busy = !m_busy;
 		m_busyEvents = events;
 		m_knownSteps = 0;

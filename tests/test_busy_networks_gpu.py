@@ -99,6 +99,19 @@ def test_nemo_step(n, form, stdp):
     same_end(a, b, n, fanout, stdp)
 
 
+def test_calm_after_a_resident_loop_of_a_very_busy_network():
+    """What the loop had counted when it was stopped, a hundred rounds a step,
+    does not weigh on the calm network later."""
+    n, fanout = 600, 390
+    a, b = (nb.Simulation(network(n, fanout, 1.0), nb.Configuration()) for _ in range(2))
+    b.set_resident_step(0)
+    assert [list(a.step()) for _ in range(70)] == [list(b.step()) for _ in range(70)]
+    assert a.step_kernel() == "run_kernel"
+    set_rates((a, b), n, 0.001)
+    assert [list(a.step()) for _ in range(200)] == [list(b.step()) for _ in range(200)]
+    assert a.step_kernel() == "local_run_kernel<1>"
+
+
 def test_two_launch_shape_of_a_large_learning_network():
     """Without a shape of the caller's, the two-launch step of a large network
     with STDP takes wider partitions while the network fires often."""
